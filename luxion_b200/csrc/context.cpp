@@ -838,6 +838,7 @@ int enqueue_wave(lux_ctx* C, int ns, const cudaEvent_t* ev) {
         ++k;
     };
     LUX_CUDA(cudaMemsetAsync(W.ctr, 0, sizeof(WaveCounters), st));
+    if (C->opt.ray_sorting) LUX_CUDA(clear_sort_counters(C->sort_temp, st));
     rec();
     LUX_CUDA(launch_camera(C->S, W, C->dopt, C->cam, n, 0, W.wave_iter, st));
     rec();
@@ -944,6 +945,12 @@ int enqueue_pipelined(lux_ctx* C, int nw, int ns_last, int h0, Spans* sp) {
     return LUX_OK;
 }
 
+// The error word of a wave's counters.
+int wave_error(int bits) {
+    if (bits & 1) return fail(LUX_ERR_UNSUPPORTED, "traversal stack overflow");
+    return fail(LUX_ERR_TIMEOUT, "a wait of the ray sort gave up");
+}
+
 // Stats of a finished call from the waves' counters and, when timed, the marked spans.
 int finish_stats(lux_ctx* C, int nwaves, int n_iter, const Spans* sp, int steps) {
     const int depth = C->dopt.trace_depth;
@@ -951,7 +958,7 @@ int finish_stats(lux_ctx* C, int nwaves, int n_iter, const Spans* sp, int steps)
     const int spw = C->spp_per_wave;
     for (int w = 0; w < nwaves; ++w) {
         const WaveCounters& c = C->h_ctr[w];
-        if (c.error) return fail(LUX_ERR_UNSUPPORTED, "traversal stack overflow");
+        if (c.error) return wave_error(c.error);
         for (int b = 0; b < depth; ++b) {
             C->stats.rays_radiance += c.count[b];
             C->stats.path_bounces += c.count[b];
@@ -1108,10 +1115,10 @@ int run_waves(lux_ctx* C, int first_iter, int n_iter) {
     C->stats.ms_total = ms;
     const int depth = C->dopt.trace_depth;
     const bool nee = C->dopt.dl || C->dopt.env;
-    const int sort_launches = 1 + 4 * 3;
+    const int sort_launches = 1 + 4;
     for (int w = 0; w < nwaves; ++w) {
         const WaveCounters& c = C->h_ctr[w];
-        if (c.error) return fail(LUX_ERR_UNSUPPORTED, "traversal stack overflow");
+        if (c.error) return wave_error(c.error);
         for (int b = 0; b < depth; ++b) {
             C->stats.rays_radiance += c.count[b];
             C->stats.path_bounces += c.count[b];

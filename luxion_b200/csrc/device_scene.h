@@ -121,7 +121,8 @@ struct DevOptions {
 //   count[b]     queue length entering bounce b (count[0] = paths of the wave)
 //   shadow[b]    shadow rays queued at bounce b
 //   fetch_r[b], fetch_s[b]  work-fetch cursors of the persistent trace kernels
-//   error        sticky error word (bit 0: traversal stack overflow)
+//   error        sticky error word (bit 0: traversal stack overflow, bit 1: a wait of the ray
+//                sort gave up)
 constexpr int kMaxDepth = 64;
 struct WaveCounters {
     int count[kMaxDepth + 1];

@@ -62,6 +62,8 @@ cudaError_t launch_convert_texels(const void* src, int fmt, int to_half, void* d
 cudaError_t launch_morton_sort(const DevScene& S, DevWave& W, int bounce, void* temp, size_t temp_bytes,
                                cudaStream_t st);
 size_t morton_sort_temp_bytes(int max_paths);
+// before the first bounce of a wave: the sort's counters start at zero
+cudaError_t clear_sort_counters(void* temp, cudaStream_t st);
 cudaError_t launch_morton_ext(const DevScene& S, const float* rays, uint32_t* keys, int n, cudaStream_t st);
 
 // kernel-level parity entry points (device buffers)
