@@ -7,7 +7,9 @@
 namespace lux {
 
 constexpr int kTraceBlock = 128;
-constexpr int kShadeBlock = 128;
+constexpr int kShadeBlock = 384;  // three blocks per SM; both measured, see k_shade
+constexpr int kShadeOcc = 3;
+constexpr int kCameraBlock = 128;
 
 // persistent traversal grid of `mode` for the two-level or the single-level layout
 int trace_grid_blocks(int mode, bool single = false);

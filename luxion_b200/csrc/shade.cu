@@ -154,12 +154,24 @@ LUX_DI Isect ch_direct_light(const DevScene& S, float t, int inst, int prim, flo
     return r;
 }
 
+// vpow in one copy of powf's code, run three times (see k_shade on why code size matters)
+LUX_DI f3 vpow_loop(f3 v, float e) {
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c) {
+        const float r = powf(v.x, e);
+        v.x = v.y;
+        v.y = v.z;
+        v.z = r;
+    }
+    return v;
+}
+
 // ---- material queries (src/material_queries.cu:19-117)
 LUX_DI f3 get_albedo(const DevMaterial& m, float u, float v) {
     if (m.flags & kMatAlbedoTex) {
         tt_apply(m.albedo_tt, u, v);
         float4 t = tex(m.albedo_tex, u, v);
-        return vpow(mk(t.x, t.y, t.z), 2.2f);
+        return vpow_loop(mk(t.x, t.y, t.z), 2.2f);
     }
     return mk(m.color[0], m.color[1], m.color[2]);
 }
@@ -202,7 +214,7 @@ LUX_DI f3 get_emission(const DevMaterial& m, float u, float v) {
     if (m.flags & kMatEmissiveTex) {
         tt_apply(m.emissive_tt, u, v);
         float4 t = tex(m.emissive_tex, u, v);
-        e = e * vpow(mk(t.x, t.y, t.z), 2.2f);
+        e = e * vpow_loop(mk(t.x, t.y, t.z), 2.2f);
     }
     return e;
 }
@@ -312,19 +324,6 @@ LUX_DI f3 BTDF(f3 wo, f3 n, f3 wi, f3 albedo, float rough, float metal, float io
     float DFG = D * G * (1.0f - F);
     return albedo * (trans * (1.0f - metal) * (cnum / cden) * jac * DFG);
 }
-// calculateRandomDirectionInHemisphere (src/interactions.cu:7-45)
-LUX_DI f3 hemisphere(f3 n, Rng& rng) {
-    float up = sqrtf(rng.u01());
-    float over = sqrtf(1.0f - up * up);
-    float around = rng.u01() * kTWO_PI;
-    f3 dnn;
-    if (fabsf(n.x) < kSQRT13) dnn = mk(1.0f, 0.0f, 0.0f);
-    else if (fabsf(n.y) < kSQRT13) dnn = mk(0.0f, 1.0f, 0.0f);
-    else dnn = mk(0.0f, 0.0f, 1.0f);
-    f3 p1 = normalize(cross(n, dnn));
-    f3 p2 = normalize(cross(n, p1));
-    return up * n + cosf(around) * over * p1 + sinf(around) * over * p2;
-}
 LUX_DI void lobe_probs(f3 wo, f3 n, float metal, f3 color, float ior, float trans, float& pR, float& pD, float& pS) {
     bool enter = dot(wo, n) > 0.0f;
     float etaI = enter ? 1.0f : ior, etaT = enter ? ior : 1.0f;
@@ -347,21 +346,37 @@ LUX_DI Lobes lobes_of(f3 wo, f3 n, float metal, f3 color, float ior, float trans
     lobe_probs(wo, n, metal, color, gmax(ior, 1.0001f), trans, L.pR, L.pD, L.pS);
     return L;
 }
-// sampleCookTorrance (src/shaders/cook_torrance.cu:156-224); L = lobes_of(wo, n, metal, color, ior, trans)
+// sampleCookTorrance (src/shaders/cook_torrance.cu:156-224) with the diffuse lobe's
+// calculateRandomDirectionInHemisphere (src/interactions.cu:7-45); L = lobes_of(wo, n, metal,
+// color, ior, trans), ior at least 1.0001. Both lobes take their angle around the axis from the
+// third draw, so one sine and cosine serve both.
 LUX_DI f3 sample_ct(f3 wo, f3 n, float rough, Rng& rng, float ior, const Lobes& L) {
-    float r = rng.u01();
-    ior = gmax(ior, 1.0001f);
+    const float r = rng.u01();
+    const float x1 = rng.u01(), x2 = rng.u01();
     rough = gclamp(rough, 0.0001f, 1.0f);
     float alpha = rough * rough;
     bool enter = dot(wo, n) > 0.0f;
     f3 nf = enter ? n : -n;
-    float etaI = enter ? 1.0f : ior, etaT = enter ? ior : 1.0f;
     const float pD = L.pD, pS = L.pS;
-    if (r > pS && r <= pS + pD) return hemisphere(nf, rng);
-    float x1 = rng.u01(), x2 = rng.u01();
+    static_assert(2.0f * kPI == kTWO_PI, "the lobes' angles around the axis");
+    float sp, cp;
+    sincosf(x2 * kTWO_PI, &sp, &cp);
+    if (r > pS && r <= pS + pD) {
+        float up = sqrtf(x1);
+        float over = sqrtf(1.0f - up * up);
+        f3 dnn;
+        if (fabsf(nf.x) < kSQRT13) dnn = mk(1.0f, 0.0f, 0.0f);
+        else if (fabsf(nf.y) < kSQRT13) dnn = mk(0.0f, 1.0f, 0.0f);
+        else dnn = mk(0.0f, 0.0f, 1.0f);
+        f3 p1 = normalize(cross(nf, dnn));
+        f3 p2 = normalize(cross(nf, p1));
+        return up * nf + cp * over * p1 + sp * over * p2;
+    }
+    float etaI = enter ? 1.0f : ior, etaT = enter ? ior : 1.0f;
     float th = atanf((alpha * sqrtf(x1)) / sqrtf(1.0f - x1));
-    float ph = 2.0f * kPI * x2;
-    f3 h = normalize(mk(1.0f * sinf(th) * cosf(ph), 1.0f * sinf(th) * sinf(ph), 1.0f * cosf(th)));
+    float st, ct;
+    sincosf(th, &st, &ct);
+    f3 h = normalize(mk(1.0f * st * cp, 1.0f * st * sp, 1.0f * ct));
     f3 t = normalize(fabsf(nf.z) < 0.999f ? cross(mk(0.0f, 0.0f, 1.0f), nf) : cross(mk(1.0f, 0.0f, 0.0f), nf));
     f3 b = cross(nf, t);
     f3 hw = h.x * t + h.y * b + h.z * nf;
@@ -403,18 +418,15 @@ LUX_DI float PDF(f3 wo, f3 wi, f3 n, float rough, float ior, const Lobes& L) {
     float pdf = refr ? L.pR * pdfR : L.pD * pdfD + L.pS * pdfS;
     return gmax(pdf, kPDF_CLAMP);
 }
-LUX_DI f3 shade_ct(f3 wo, f3 albedo, f3 n, f3 wi, float rough, float metal, float ior, float trans) {
-    ior = gmax(ior, 1.0001f);
-    bool refr = (dot(wi, n) * dot(wo, n)) < 0.0f;
-    f3 f = refr ? BTDF(wo, n, wi, albedo, rough, metal, ior, trans) : BRDF(wo, n, wi, albedo, rough, metal, ior, trans);
-    return f * fabsf(dot(wi, n));
-}
 
 // ---- environment (src/kernels/shade_path.cu:27-42, :207-215)
-LUX_DI float envmap_pdf(const DevScene& S, f3 d) {
+// Spherical coordinates of a direction, as both the pdf and the lookup take them.
+LUX_DI void env_angles(f3 d, float& phi, float& theta) {
+    phi = atan2f(d.z, d.x);
+    theta = acosf(gclamp(d.y, -1.0f, 1.0f));
+}
+LUX_DI float envmap_pdf(const DevScene& S, float phi, float theta) {
     const int W = S.env_w, H = S.env_h;
-    float phi = atan2f(d.z, d.x);
-    float theta = acosf(gclamp(d.y, -1.0f, 1.0f));
     float u = (phi + kPI) / (2.0f * kPI);
     float v = theta / kPI;
     int col = gclampi(int(u * float(W)), 0, W - 1);
@@ -425,9 +437,7 @@ LUX_DI float envmap_pdf(const DevScene& S, f3 d) {
     float st = sinf(theta);
     return (st > 1e-6f) ? (pm * pc) / (2.0f * kPI * kPI * st) : 0.0f;
 }
-LUX_DI f3 env_lookup(const DevScene& S, f3 d, float intensity) {
-    float phi = atan2f(d.z, d.x);
-    float theta = acosf(gclamp(d.y, -1.0f, 1.0f));
+LUX_DI f3 env_lookup(const DevScene& S, float phi, float theta, float intensity) {
     float u = float((double(phi) + kM_PI_SHADE) * (double(1.0f) / (double(2.0f) * kM_PI_SHADE)));
     float v = float(double(theta) * (double(1.0f) / kM_PI_SHADE));
     float4 e = tex(S.env_tex, u, v);
@@ -490,9 +500,10 @@ LUX_DI f3 light_sample(const DevScene& S, const DevOptions& O, int iter, int pix
         float u = (float(cn) + 0.5f) / float(W);
         float v = (float(mg) + 0.5f) / float(H);
         float phi = float(double(u) * 2.0 * double(kPI) - double(kPI));
-        float theta = v * kPI;
-        float st = sinf(theta);
-        env_dir = mk(st * cosf(phi), cosf(theta), st * sinf(phi));
+        float st, ct, sp, cp;
+        sincosf(v * kPI, &st, &ct);
+        sincosf(phi, &sp, &cp);
+        env_dir = mk(st * cp, ct, st * sp);
     }
     return dl;
 }
@@ -517,6 +528,12 @@ struct WavePathIn {
     LUX_DI f3 nee() const { float4 a = ld_stream(&W.s4[pid]); return mk(a.x, a.y, a.z); }
 };
 
+// A phase boundary of the shading: the block's warps meet, so that they fetch the next phase's
+// instructions together (k_shade).
+template <bool PHASED> LUX_DI void phase() {
+    if (PHASED) __syncthreads();
+}
+
 // shadePath for one path; returns true if the path survives (is not killed).
 // sh_t: DL shadow hit t (or env occlusion); sh_* the DL shadow hit record.
 // MATDBG: the instantiation that also renders the material debug views (O.material_debug).
@@ -526,20 +543,35 @@ struct WavePathIn {
 // hit kills, as the reference does (its result is then unused; the parity entry reports it).
 // The NEE terms draw no random numbers, so sampling the direction after them leaves the
 // random stream as the reference's (sample first, then Russian roulette).
-template <bool MATDBG, int NEE, bool SPAWN_KILLED, class In>
+//
+// The shading runs in steps that every path of the warp takes part in, hit or miss, each step in
+// one copy of its code: surface, light (emission, shadow result, environment), then the BSDF for
+// the light's direction and for the sampled one. Paths that end in the environment share the
+// environment step with the hits that sample it, and the two BSDF evaluations of a hit share
+// theirs. on: false for a lane that only takes part in the phases (PHASED needs every thread of
+// the block; the results of such a lane are not read).
+template <bool MATDBG, int NEE, bool SPAWN_KILLED, bool PHASED, class In>
 LUX_DI bool shade_one(const DevScene& S, const DevOptions& O, int depth, PathState& p, const In& in, float t, int inst,
-                      int prim, float bu, float bv, float sh_t, int sh_inst, int sh_prim, float sh_u, float sh_v) {
+                      int prim, float bu, float bv, float sh_t, int sh_inst, int sh_prim, float sh_u, float sh_v,
+                      bool on = true) {
     Rng rng = Rng::seeded(p.iter, p.pixel, depth);
     f3 add = mk(0.0f, 0.0f, 0.0f);
     bool added = false;
     const bool has_exr = S.has_env != 0;
-    bool kill = false;
-    if (inst >= 0 && t > 0.0f) {
-        Isect is = ch_radiance(S, t, inst, prim, bu, bv);
+    const bool hit = on && inst >= 0 && t > 0.0f;
+    const bool miss = on && !hit;
+    const f3 wo = -p.d;
+    // ---- surface
+    f3 mc, normal, n0, emission;
+    float rough = 0.0f, metal = 0.0f, ior = 1.0f, trans = 0.0f;
+    bool emissive = false;
+    mc = normal = n0 = emission = mk(0.0f, 0.0f, 0.0f);
+    if (hit) {
+        const Isect is = ch_radiance(S, t, inst, prim, bu, bv);
         const DevMaterial& m = S.mats[is.material];
-        f3 mc = get_albedo(m, is.u, is.v);
-        f3 normal = get_normal(S, m, is);
-        float rough, metal;
+        mc = get_albedo(m, is.u, is.v);
+        normal = get_normal(S, m, is);
+        n0 = is.normal;
         get_mr(m, is.u, is.v, rough, metal);
         if (MATDBG && O.material_debug) {
             // the debug view replaces the colour and ends the path (shade_path.cu:154-164)
@@ -547,126 +579,153 @@ LUX_DI bool shade_one(const DevScene& S, const DevOptions& O, int depth, PathSta
                                            get_alpha(m, is.u, is.v));
             return false;
         }
-        f3 emission = get_emission(m, is.u, is.v);
-        bool is_spec = rough < kSPEC_ROUGH;
-        f3 nf = dot(-p.d, normal) < 0.0f ? -normal : normal;
-        const float ior = m.ior, trans = m.transmission;
-        bool emissive = length(emission) > kEPS_UTIL;
-        const Lobes L = lobes_of(-p.d, normal, metal, mc, ior, trans);
-        if (nee_env<NEE>(O)) {
-            if (emissive) {
-                float w = 1.0f;
-                if (depth > 1 && !p.spec) {
-                    float pb = in.last_pdf();
-                    float pe = envmap_pdf(S, p.d);
-                    w = (pb * pb) / (pb * pb + pe * pe);
-                }
-                add = p.thr * (w * emission);
-                added = true;
-                kill = true;
-            } else if (sh_t < 0.0f && !is_spec && has_exr) {
-                f3 ed = in.nee();
-                float pee = envmap_pdf(S, ed);
-                float pbe = PDF(-p.d, ed, normal, rough, ior, L);
-                float w = (pee * pee) / (pee * pee + pbe * pbe);
-                f3 brdf = BRDF(-p.d, normal, ed, mc, rough, metal, ior, trans);
-                f3 el = env_lookup(S, normalize(ed), O.env_intensity);
-                float cs = dot(nf, ed);
-                if (cs > 0.0f && pee > 1e-8f) {
-                    f3 contrib = (el * brdf * cs) / pee;
-                    add = p.thr * contrib * w;
-                    added = true;
-                }
-            }
-        } else if (nee_dl<NEE>(O)) {
-            if (emissive) {
-                float w = 1.0f;
-                if (depth > 1 && !p.spec) {
-                    float pb = in.last_pdf();
-                    float dsq = is.t * is.t;
-                    float cl = dot(is.normal, -p.d);
-                    if (cl > 0.0001f) {
-                        float pa = 1.0f / S.total_area;
-                        float ps = pa * (dsq / cl);
-                        w = (pb * pb) / (pb * pb + ps * ps);
-                    } else {
-                        w = 0.0f;
+        emission = get_emission(m, is.u, is.v);
+        emissive = length(emission) > kEPS_UTIL;
+        ior = gmax(m.ior, 1.0001f);
+        trans = m.transmission;
+    }
+    phase<PHASED>();
+    const bool is_spec = rough < kSPEC_ROUGH;
+    const f3 nf = dot(wo, normal) < 0.0f ? -normal : normal;
+    // MIS applies to the light a BSDF sample found (not for camera rays and specular bounces)
+    const bool mis = depth > 1 && !p.spec;
+    const bool kill_light = hit && emissive;
+    // ---- light: pl, le, cs are the light sample's pdf, radiance and cosine, wl its direction,
+    // for hits whose sample is visible (lit)
+    bool lit = false;
+    f3 wl = mk(0.0f, 0.0f, 0.0f), le = wl;
+    float pl = 0.0f, cs = 0.0f;
+    float w = 1.0f;  // MIS weight of emission or the environment found by the BSDF
+    if (nee_env<NEE>(O)) {
+        if (hit && !emissive && sh_t < 0.0f && !is_spec && has_exr) {
+            wl = in.nee();
+            cs = dot(nf, wl);
+            lit = cs > 0.0f;  // a sample below the horizon contributes nothing
+        }
+    }
+    if (has_exr && (miss || (hit && nee_env<NEE>(O)))) {
+        const f3 dm = hit ? p.d : normalize(p.d);
+        f3 d = lit ? wl : dm;
+        bool pdf = lit || (nee_env<NEE>(O) && mis && (!hit || emissive));
+        bool look = !hit && !pdf;
+        // a hit's sample takes the pdf of its direction and the radiance of the normalised one;
+        // a miss takes both of one direction
+        if (pdf || look) {
+#pragma unroll 1
+            while (true) {
+                float phi, theta;
+                env_angles(d, phi, theta);
+                if (pdf) {
+                    pl = envmap_pdf(S, phi, theta);
+                    pdf = false;
+                    if (lit && pl > 1e-8f) {
+                        d = normalize(wl);
+                        look = true;
+                        continue;
                     }
+                    look = !hit;
                 }
-                add = p.thr * (w * emission);
-                added = true;
-                kill = true;
-            } else if (sh_inst >= 0 && sh_t > 0.0f && !is_spec) {
-                Isect dli = ch_direct_light(S, sh_t, sh_inst, sh_prim, sh_u, sh_v);
-                f3 sp = is.t * p.d + in.origin();
-                f3 lv = in.nee() - sp;
-                float dsq = dot(lv, lv);
-                float dist = sqrtf(dsq);
-                f3 ld = lv / dist;
-                float cs = dot(nf, ld);
-                float cl = dot(dli.normal, -ld);
-                if (cs > 0.0f && cl > 0.0f) {
+                if (look) le = env_lookup(S, phi, theta, O.env_intensity);
+                break;
+            }
+        }
+        if (lit) lit = pl > 1e-8f;
+        else if (mis && (nee_env<NEE>(O)) && (!hit || emissive)) {
+            const float pb = in.last_pdf();
+            w = (pb * pb) / (pb * pb + pl * pl);
+        }
+    }
+    if (nee_dl<NEE>(O) && !nee_env<NEE>(O) && hit) {
+        if (emissive) {
+            if (mis) {
+                float pb = in.last_pdf();
+                float dsq = t * t;
+                float cl = dot(n0, wo);
+                if (cl > 0.0001f) {
                     float pa = 1.0f / S.total_area;
                     float ps = pa * (dsq / cl);
-                    float pb = PDF(-p.d, ld, normal, rough, ior, L);
-                    float w = (ps * ps) / (ps * ps + pb * pb);
-                    f3 brdf = BRDF(-p.d, normal, ld, mc, rough, metal, ior, trans);
-                    const DevMaterial& lm = S.mats[dli.material];
-                    f3 lr = get_emission(lm, dli.u, dli.v);
-                    f3 contrib = (lr * brdf * cs) / ps;
-                    add = p.thr * contrib * w;
-                    added = true;
+                    w = (pb * pb) / (pb * pb + ps * ps);
+                } else {
+                    w = 0.0f;
                 }
             }
-        } else if (emissive) {
-            add = p.thr * emission;
-            added = true;
-            kill = true;
-        }
-        if (kill && !SPAWN_KILLED) {
-            p.color = in.color0() + add;
-            return false;
-        }
-        f3 sd = sample_ct(-p.d, normal, rough, rng, ior, L);
-        if (!kill) {
-            bool transmitted = dot(-p.d, normal) * dot(sd, normal) < 0.0f;
-            bool spec = is_spec || transmitted;
-            f3 f = shade_ct(-p.d, mc, normal, sd, rough, metal, ior, trans);
-            float pdf = PDF(-p.d, sd, normal, rough, ior, L);
-            p.thr = p.thr * (f / pdf);
-            p.last_pdf = pdf;
-            p.spec = spec;
-            if (depth >= kRR_MIN_DEPTH) {
-                float mx = gmax(p.thr.x, gmax(p.thr.y, p.thr.z));
-                float surv = gclamp(mx, 0.0f, 1.0f);
-                if (rng.u01() >= surv) kill = true;
-                else p.thr = p.thr / surv;
+        } else if (sh_inst >= 0 && sh_t > 0.0f && !is_spec) {
+            Isect dli = ch_direct_light(S, sh_t, sh_inst, sh_prim, sh_u, sh_v);
+            f3 sp = t * p.d + in.origin();
+            f3 lv = in.nee() - sp;
+            float dsq = dot(lv, lv);
+            float dist = sqrtf(dsq);
+            wl = lv / dist;
+            cs = dot(nf, wl);
+            float cl = dot(dli.normal, -wl);
+            if (cs > 0.0f && cl > 0.0f) {
+                float pa = 1.0f / S.total_area;
+                pl = pa * (dsq / cl);
+                const DevMaterial& lm = S.mats[dli.material];
+                le = get_emission(lm, dli.u, dli.v);
+                lit = true;
             }
         }
-        p.color = added ? in.color0() + add : in.color0();
-        // ray spawn (shade_path.cu:333-353), run for paths killed above as well
-        f3 hp = in.origin() + (is.t - .0001f) * normalize(p.d);
-        float sl2 = dot(sd, sd);
-        if (!(sl2 > 1e-12f) || !isfinite(sl2)) return false;
-        p.d = sd;
-        if (dot(p.d, is.normal) > 0.0f) p.o = hp + (is.normal * kGLASS_EPS);
-        else p.o = hp - (is.normal * kGLASS_EPS);
-        return !kill;
     }
-    if (has_exr) {
-        f3 d = normalize(p.d);
-        f3 er = env_lookup(S, d, O.env_intensity);
-        float w = 1.0f;
-        if (nee_env<NEE>(O) && depth > 1 && !p.spec) {
-            float pb = in.last_pdf();
-            float pe = envmap_pdf(S, d);
-            w = (pb * pb) / (pb * pb + pe * pe);
+    phase<PHASED>();
+    bool kill = kill_light;
+    bool done = !hit;  // no BSDF step: a miss, or an emitter hit whose ray is not spawned
+    if (miss) {
+        if (has_exr) {
+            add = p.thr * le * w;
+            added = true;
         }
-        add = p.thr * er * w;
+    } else if (hit && emissive) {
+        add = (nee_env<NEE>(O) || nee_dl<NEE>(O)) ? p.thr * (w * emission) : p.thr * emission;
         added = true;
+        done = !SPAWN_KILLED;
     }
-    p.color = added ? in.color0() + add : in.color0();
-    return false;
+    // ---- BSDF: k = 0 for the light's direction, k = 1 for the sampled one
+    Lobes L;
+    L.pR = L.pD = L.pS = 0.0f;
+    if (!done) L = lobes_of(wo, normal, metal, mc, ior, trans);
+    f3 sd = mk(0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+    for (int k = NEE == 0 ? 1 : 0; k < 2; ++k) {
+        if (k == 1) {
+            if (!done) sd = sample_ct(wo, normal, rough, rng, ior, L);
+            phase<PHASED>();
+        }
+        if (!(done || (k == 0 ? !lit : kill))) {
+            const f3 wi = k == 0 ? wl : sd;
+            const bool refr = (dot(wi, normal) * dot(wo, normal)) < 0.0f;
+            const float pdf = PDF(wo, wi, normal, rough, ior, L);
+            const f3 f = (k == 1 && refr) ? BTDF(wo, normal, wi, mc, rough, metal, ior, trans)
+                                          : BRDF(wo, normal, wi, mc, rough, metal, ior, trans);
+            if (k == 0) {
+                const float wt = (pl * pl) / (pl * pl + pdf * pdf);
+                f3 contrib = (le * f * cs) / pl;
+                add = p.thr * contrib * wt;
+                added = true;
+            } else {
+                p.thr = p.thr * ((f * fabsf(dot(wi, normal))) / pdf);
+                p.last_pdf = pdf;
+                p.spec = is_spec || refr;
+                if (depth >= kRR_MIN_DEPTH) {
+                    float mx = gmax(p.thr.x, gmax(p.thr.y, p.thr.z));
+                    float surv = gclamp(mx, 0.0f, 1.0f);
+                    if (rng.u01() >= surv) kill = true;
+                    else p.thr = p.thr / surv;
+                }
+            }
+        }
+        phase<PHASED>();
+    }
+    if (on) p.color = added ? in.color0() + add : in.color0();
+    if (done) return false;
+    // ray spawn (shade_path.cu:333-353), run for paths killed above as well
+    f3 hp = in.origin() + (t - .0001f) * normalize(p.d);
+    float sl2 = dot(sd, sd);
+    if (!(sl2 > 1e-12f) || !isfinite(sl2)) return false;
+    p.d = sd;
+    if (dot(p.d, n0) > 0.0f) p.o = hp + (n0 * kGLASS_EPS);
+    else p.o = hp - (n0 * kGLASS_EPS);
+    return !kill;
 }
 
 // The fields shade_one reads on entry.
@@ -700,7 +759,7 @@ LUX_HDI int tiled_pixel(int t, int W, int H) {
 }
 
 // Paths [0, n) of a wave in lane `lane`: path ids and queue slots from lane * lane_stride on.
-__global__ void __launch_bounds__(kShadeBlock, 16) k_camera(DevScene S, DevWave W, DevOptions O, DevCamera C, int n,
+__global__ void __launch_bounds__(kCameraBlock, 16) k_camera(DevScene S, DevWave W, DevOptions O, DevCamera C, int n,
                                                             int lane, const int* wave_iter) {
     const int first_iter = wave_iter[0];
     const bool nee = O.dl || O.env;
@@ -734,14 +793,18 @@ __global__ void __launch_bounds__(kShadeBlock, 16) k_camera(DevScene S, DevWave 
 
 // JOBS: the shared wavefront of the job engine; each path shades against its job's scene
 // (lights, environment) and stops compacting at its job's trace depth.
-// Full occupancy (16 blocks of 128 threads per SM, 32 registers): the kernel waits mostly on
-// texture fetches and gathers, and hiding that latency with more warps pays more than the
-// register spills cost (shade per 16-spp step of the 1M-triangle 1080p workload: 28.3 ms at
-// 5 blocks per SM, 22.6 at 8, 20.4 at 12, 18.8 at 16).
+// The code of one path is some 5000 instructions with little reuse, far more than an SM's
+// instruction caches hold, so warps that run at their own pace starve on instruction fetch (with
+// 16 free-running 128-thread blocks per SM: 14.0 of 31 stall cycles per issue, bounce 1 of the
+// 1M-triangle 1080p scene). Here the warps of a block walk the phases of shade_one in step and
+// share each fetched line: 0.3 stall cycles, and what is left is waiting for loads (12 of 24).
+// Shade time of that scene's 16-spp step: 12.95 ms free-running; in step with 128-thread blocks
+// 13.7, 256 x 8 per SM 13.0, 512 x 4 12.2, 512 x 3 (40 registers) 11.0, 384 x 3 (56) 10.7,
+// 256 x 4 (64) 11.0, 512 x 2 (64) 11.8, 1024 x 1 11.9.
 // G: the (lane, bounce) segments of waves in flight this launch shades; the paths of segment k
 // are its lane's queue at its bounce, and its survivors go to the lane's next queue.
 template <bool JOBS, bool MATDBG, int NEE>
-__global__ void __launch_bounds__(kShadeBlock, 16) k_shade(const __grid_constant__ DevScene S0, DevWave W, DevOptions O,
+__global__ void __launch_bounds__(kShadeBlock, kShadeOcc) k_shade(const __grid_constant__ DevScene S0, DevWave W, DevOptions O,
                                                        const __grid_constant__ Segs G) {
     __shared__ int seg_first[kMaxSegs + 1];
     if (threadIdx.x == 0) {
@@ -756,32 +819,36 @@ __global__ void __launch_bounds__(kShadeBlock, 16) k_shade(const __grid_constant
     const int n = seg_first[kMaxSegs];
     const bool nee = nee_dl<NEE>(O) || nee_env<NEE>(O);
     const int lane = threadIdx.x & 31;
-    const int stride = gridDim.x * blockDim.x;
-    // uniform trip count across the warp so the append below runs converged
-    for (int base = blockIdx.x * blockDim.x; base < n; base += stride) {
+    // A launch of fewer paths than the grid has threads gives every block its share, in whole
+    // warps, so that they reach all SMs.
+    const int chunk = min(kShadeBlock, ((n + int(gridDim.x) - 1) / int(gridDim.x) + 31) & ~31);
+    const int stride = int(gridDim.x) * chunk;
+    // uniform trip count across the block: the phases run in step
+    for (int base = blockIdx.x * chunk; base < n; base += stride) {
         const int item = base + threadIdx.x;
+        const bool on = int(threadIdx.x) < chunk && item < n;
         bool alive = false;
-        int pid = 0, k = 0;
-        if (item < n) {
+        int pid = 0, k = 0, depth = 0, job_compact = 0;
+        const DevScene* sp = &S0;
+        PathState p{};
+        float4 h = make_float4(-1.0f, 0.0f, 0.0f, __int_as_float(-1));
+        int prim = 0, si = -1, spr = -1;
+        float sh_t = -1.0f, su = 0.0f, sv = 0.0f;
+        if (on) {
             while (k + 1 < G.n && item >= seg_first[k + 1]) ++k;
             const int slot = G.lane[k] * W.lane_stride + (item - seg_first[k]);
-            const int depth = G.bounce[k] + 1;
+            depth = G.bounce[k] + 1;
             pid = ld_stream(&W.queue[G.bounce[k] & 1][slot]);
-            int job_compact = G.compact[k];
-            const DevScene* sp = &S0;
+            job_compact = G.compact[k];
             if (JOBS) {
                 const DevJob& J = W.jobs[W.path_job[pid]];
                 sp = &W.scenes[J.scene];
                 job_compact = depth < J.trace_depth;
             }
-            const DevScene& S = *sp;
-            PathState p = load_path(W, pid);
-            float4 h = ld_stream(&W.hit[slot]);
-            int inst = __float_as_int(h.w);
-            int prim = ld_stream(&W.hit_prim[slot]);
-            float sh_t = -1.0f, su = 0.0f, sv = 0.0f;
-            int si = -1, spr = -1;
-            if (nee && inst >= 0) {
+            p = load_path(W, pid);
+            h = ld_stream(&W.hit[slot]);
+            prim = ld_stream(&W.hit_prim[slot]);
+            if (nee && __float_as_int(h.w) >= 0) {
                 float4 sh = ld_stream(&W.sh_hit[slot]);
                 sh_t = sh.x;
                 if (!nee_env<NEE>(O)) {
@@ -791,20 +858,21 @@ __global__ void __launch_bounds__(kShadeBlock, 16) k_shade(const __grid_constant
                     spr = ld_stream(&W.sh_prim[slot]);
                 }
             }
-            alive = shade_one<MATDBG, NEE, false>(S, O, depth, p, WavePathIn{W, pid}, h.x, inst, prim, h.y, h.z, sh_t, si, spr,
-                                           su, sv) &&
-                    job_compact;
-            st_stream(&W.s3[pid], make_float4(p.color.x, p.color.y, p.color.z, __int_as_float(p.iter)));
-            if (alive) {
-                st_stream(&W.s0[pid], make_float4(p.o.x, p.o.y, p.o.z, p.last_pdf));
-                st_stream(&W.s1[pid], make_float4(p.d.x, p.d.y, p.d.z, __int_as_float(p.spec ? 1 : 0)));
-                st_stream(&W.s2[pid], make_float4(p.thr.x, p.thr.y, p.thr.z, __int_as_float(p.pixel)));
-                if (nee) {
-                    f3 ed;
-                    f3 dl = light_sample<NEE>(S, O, p.iter, p.pixel, depth, ed, !nee_env<NEE>(O));
-                    f3 v = nee_env<NEE>(O) ? ed : dl;
-                    st_stream(&W.s4[pid], make_float4(v.x, v.y, v.z, 0.0f));
-                }
+        }
+        const DevScene& S = *sp;
+        alive = shade_one<MATDBG, NEE, false, !MATDBG>(S, O, depth, p, WavePathIn{W, pid}, h.x, __float_as_int(h.w), prim,
+                                                      h.y, h.z, sh_t, si, spr, su, sv, on) &&
+                job_compact;
+        if (on) st_stream(&W.s3[pid], make_float4(p.color.x, p.color.y, p.color.z, __int_as_float(p.iter)));
+        if (alive) {
+            st_stream(&W.s0[pid], make_float4(p.o.x, p.o.y, p.o.z, p.last_pdf));
+            st_stream(&W.s1[pid], make_float4(p.d.x, p.d.y, p.d.z, __int_as_float(p.spec ? 1 : 0)));
+            st_stream(&W.s2[pid], make_float4(p.thr.x, p.thr.y, p.thr.z, __int_as_float(p.pixel)));
+            if (nee) {
+                f3 ed;
+                f3 dl = light_sample<NEE>(S, O, p.iter, p.pixel, depth, ed, !nee_env<NEE>(O));
+                f3 v = nee_env<NEE>(O) ? ed : dl;
+                st_stream(&W.s4[pid], make_float4(v.x, v.y, v.z, 0.0f));
             }
         }
         // warp-aggregated survivor append (src/kernels/shade_path.cu:355-363), one atomic per
@@ -881,7 +949,7 @@ LUX_DI int find_segment(const DevSegment* segs, int nsegs, int v) {
 // per job): path pid belongs to the segment covering it; its sample s and pixel index give the
 // job-local iteration and pixel that seed the RNG, exactly as a single-job render would.
 // W.segs and W.wave_hdr are the wave's own tables; its paths go to lane `lane`.
-__global__ void __launch_bounds__(kShadeBlock) k_camera_jobs(DevWave W, DevOptions O, int lane) {
+__global__ void __launch_bounds__(kCameraBlock) k_camera_jobs(DevWave W, DevOptions O, int lane) {
     __shared__ DevSegment segs[kMaxSegments];
     const int nsegs = W.wave_hdr[0], n = min(W.wave_hdr[1], W.lane_stride);
     for (int k = threadIdx.x; k < nsegs; k += blockDim.x) segs[k] = W.segs[k];
@@ -1037,7 +1105,7 @@ __global__ void k_shade_ext(DevScene S, DevOptions O, float* paths, const uint32
             float su = __uint_as_float(h[8]), sv = __uint_as_float(h[9]);
             int si = int(h[6]), spr = int(h[7]);
             if (O.env) si = -1;
-            bool survived = shade_one<true, -1, true>(S, O, depth, p, RowPathIn{f, O.env != 0}, t, inst, prim,
+            bool survived = shade_one<true, -1, true, false>(S, O, depth, p, RowPathIn{f, O.env != 0}, t, inst, prim,
                                                 __uint_as_float(h[3]), __uint_as_float(h[4]), __uint_as_float(h[5]), si,
                                                 spr, su, sv);
             alive = survived && compact;
@@ -1106,12 +1174,16 @@ int shade_grid_blocks() {
     return cached;
 }
 
+// Grid cap of the camera kernels: two rounds of sixteen blocks on every SM (the shading grid is
+// three blocks an SM)
+static int camera_grid_blocks() { return shade_grid_blocks() / kShadeOcc * 32; }
+
 cudaError_t launch_camera(const DevScene& S, const DevWave& W, const DevOptions& O, const DevCamera& C, int n,
                           int lane, const int* wave_iter, cudaStream_t st) {
     if (n > W.lane_stride || lane < 0) return cudaErrorInvalidValue;
-    int grid = std::min((n + kShadeBlock - 1) / kShadeBlock, shade_grid_blocks() * 2);
+    int grid = std::min((n + kCameraBlock - 1) / kCameraBlock, camera_grid_blocks());
     if (grid < 1) grid = 1;
-    k_camera<<<grid, kShadeBlock, 0, st>>>(S, W, O, C, n, lane, wave_iter);
+    k_camera<<<grid, kCameraBlock, 0, st>>>(S, W, O, C, n, lane, wave_iter);
     return cudaGetLastError();
 }
 
@@ -1140,9 +1212,9 @@ cudaError_t launch_shade_segs(const DevScene& S, const DevWave& W, const DevOpti
 
 cudaError_t launch_camera_jobs(const DevWave& W, const DevOptions& O, int max_paths, int lane, cudaStream_t st) {
     if (lane < 0) return cudaErrorInvalidValue;
-    int grid = std::min((max_paths + kShadeBlock - 1) / kShadeBlock, shade_grid_blocks() * 2);
+    int grid = std::min((max_paths + kCameraBlock - 1) / kCameraBlock, camera_grid_blocks());
     if (grid < 1) grid = 1;
-    k_camera_jobs<<<grid, kShadeBlock, 0, st>>>(W, O, lane);
+    k_camera_jobs<<<grid, kCameraBlock, 0, st>>>(W, O, lane);
     return cudaGetLastError();
 }
 
@@ -1172,8 +1244,8 @@ cudaError_t launch_tonemap(const float* image, uint8_t* rgba, int npix, float it
 
 cudaError_t launch_shade_ext(const DevScene& S, const DevOptions& O, float* paths, const uint32_t* hits, int n,
                              int iter, int depth, int compact, int* survivors, int* n_out, cudaStream_t st) {
-    int grid = std::max(1, std::min((n + kShadeBlock - 1) / kShadeBlock, 1024));
-    k_shade_ext<<<grid, kShadeBlock, 0, st>>>(S, O, paths, hits, n, iter, depth, compact, survivors, n_out);
+    int grid = std::max(1, std::min((n + 127) / 128, 1024));
+    k_shade_ext<<<grid, 128, 0, st>>>(S, O, paths, hits, n, iter, depth, compact, survivors, n_out);
     return cudaGetLastError();
 }
 
