@@ -288,7 +288,9 @@ typedef struct lux_stats {
     double kernel_launches;   /* every kernel this library launched in the call              */
 } lux_stats;
 
-/* Per-kernel CUDA-event timing is recorded only while enabled (off by default). */
+/* Per-kernel CUDA-event timing is recorded only while enabled (off by default). A timed call runs
+ * every bounce as separate launches; an untimed one may finish few paths in one launch over all
+ * their bounces (counted in launches_trace). Images and ray counts are the same. */
 int lux_enable_timing(lux_ctx* ctx, int on);
 int lux_get_stats(lux_ctx* ctx, lux_stats* out);
 

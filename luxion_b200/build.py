@@ -7,6 +7,7 @@ Translation units:
   trace.cu    traversal kernels, FMA contraction on (exact steps use __f*_rn intrinsics)
   shade.cu    camera / shade / accumulate kernels, --fmad=false so every float op is
               rounded on its own, in the reference's order
+  paths.cu    all bounces of a path in one launch, for few paths; --fmad=false
   sort.cu     Morton keys and the radix sort of a bounce queue
   trace_static.cu  the fixed device scratch of lux_trace_rays_static
   texconv.cu  texel conversion (8/16-bit to float or binary16) at scene upload
@@ -37,6 +38,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_UNITS = {
     "trace.cu": ["--fmad=true"],
     "shade.cu": ["--fmad=false"],
+    "paths.cu": ["--fmad=false"],
     "sort.cu": ["--fmad=true"],
     "trace_static.cu": ["--fmad=true"],
     "bvh_gpu.cu": ["--fmad=false"],

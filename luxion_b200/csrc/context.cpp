@@ -825,6 +825,42 @@ int alloc_wave(lux_ctx* C, int max_paths, int lanes) {
     return LUX_OK;
 }
 
+// Whether the context's paths may be finished by the whole-path kernel: not under ray sorting
+// (the queue of every bounce is sorted), in the debug views, or in timed calls, which time the
+// kernels of each bounce apart.
+bool whole_paths(const lux_ctx* C) {
+    return !C->opt.ray_sorting && !C->opt.debug_bvh && !C->dopt.material_debug && !C->timing;
+}
+// Waves of at most kWholePerLane paths per lane of the whole-path kernel's grid (284k on 148 SMs)
+// run in it from the camera on. Above, the wavefront's full warps win: 0.81 against 1.18 ms for
+// 228k paths (477k triangles) and 0.35 against 0.53 for 66k (Cornell box), but 1.65 against 1.12 ms
+// for 367k (842k triangles). A larger wave hands over before one of the bounces 1 to kTailLast once
+// at most kTailPerLane paths per lane are left (114k) and two bounces or more are to come: a frame
+// of 2.07M paths, 1M triangles, depth 12 takes 4.18 ms instead of 5.34, while handing over at
+// twice that many took 5 to 20 % longer in 700k-triangle scenes. An attempt that finds more paths
+// left costs an empty launch.
+constexpr int kWholePerLane = 5;
+constexpr int kTailPerLane = 2;
+constexpr int kTailLast = 3;
+int path_limit(int per_lane) { return per_lane * path_grid_blocks() * kPathBlock; }
+int tail_attempts(int depth) { return std::max(0, std::min(kTailLast, depth - 2)); }
+bool try_tail(int bounce, int depth) { return bounce >= 1 && bounce <= kTailLast && bounce + 2 <= depth; }
+
+// Launches of one wave of n paths (enqueue_wave) added to the call's statistics.
+void count_launches(lux_ctx* C, int n) {
+    const int depth = C->dopt.trace_depth;
+    const bool nee = C->dopt.dl || C->dopt.env, paths = whole_paths(C);
+    C->stats.launches_camera += 1;
+    C->stats.launches_accum += 1;
+    if (paths && n <= path_limit(kWholePerLane)) {
+        C->stats.launches_trace += 1;
+        return;
+    }
+    C->stats.launches_trace += depth * (nee ? 2 : 1) + (paths ? tail_attempts(depth) : 0);
+    C->stats.launches_shade += depth;
+    C->stats.launches_sort += C->opt.ray_sorting ? depth * kSortLaunches : 0;
+}
+
 // Enqueue one wave of ns samples starting at iteration W.wave_iter[0].
 int enqueue_wave(lux_ctx* C, int ns, const cudaEvent_t* ev) {
     cudaStream_t st = C->stream;
@@ -842,7 +878,15 @@ int enqueue_wave(lux_ctx* C, int ns, const cudaEvent_t* ev) {
     rec();
     LUX_CUDA(launch_camera(C->S, W, C->dopt, C->cam, n, 0, W.wave_iter, st));
     rec();
+    const bool paths = whole_paths(C);
+    if (paths && n <= path_limit(kWholePerLane)) {
+        LUX_CUDA(launch_paths(C->S, W, C->dopt, one_seg(0), depth, n, st));
+        LUX_CUDA(launch_accumulate(W, 0, C->image, C->comp, ns, C->opt.precision == LUX_PRECISION_COMPENSATED, st));
+        return LUX_OK;
+    }
     for (int b = 0; b < depth; ++b) {
+        if (paths && try_tail(b, depth))
+            LUX_CUDA(launch_paths(C->S, W, C->dopt, one_seg(b), depth, path_limit(kTailPerLane), st));
         if (C->opt.ray_sorting) LUX_CUDA(launch_morton_sort(C->S, W, b, C->sort_temp, C->sort_temp_bytes, st));
         rec();
         if (C->opt.debug_bvh) {
@@ -926,6 +970,9 @@ int enqueue_pipelined(lux_ctx* C, int nw, int ns_last, int h0, Spans* sp) {
             G.compact[G.n] = (b + 1) < D ? 1 : 0;
             ++G.n;
         }
+        // the last wave's deep bounces have no later wave to ride along with
+        if (whole_paths(C) && t >= (nw - 1) * P && try_tail(t - (nw - 1) * P, D))
+            LUX_CUDA(launch_paths(C->S, W, C->dopt, G, D, path_limit(kTailPerLane), st));
         LUX_CUDA(launch_trace_segs(C->S, W, G, 0, nee, st));
         if (nee) LUX_CUDA(launch_trace_segs(C->S, W, G, nee == 2 ? 2 : 1, 0, st));
         if (sp) if (int rc_ = sp->mark(kSpanTrace)) return rc_;
@@ -969,7 +1016,7 @@ int finish_stats(lux_ctx* C, int nwaves, int n_iter, const Spans* sp, int steps)
     }
     C->stats.launches_camera += nwaves;
     C->stats.launches_accum += nwaves;
-    C->stats.launches_trace += steps * (nee ? 2 : 1);
+    C->stats.launches_trace += steps * (nee ? 2 : 1) + (whole_paths(C) ? tail_attempts(depth) : 0);
     C->stats.launches_shade += steps;
     if (sp) {
         for (size_t i = 1; i < sp->marks.size(); ++i) {
@@ -1114,8 +1161,6 @@ int run_waves(lux_ctx* C, int first_iter, int n_iter) {
     cudaEventElapsedTime(&ms, C->ev[0], C->ev[1]);
     C->stats.ms_total = ms;
     const int depth = C->dopt.trace_depth;
-    const bool nee = C->dopt.dl || C->dopt.env;
-    const int sort_launches = 1 + 4;
     for (int w = 0; w < nwaves; ++w) {
         const WaveCounters& c = C->h_ctr[w];
         if (c.error) return wave_error(c.error);
@@ -1126,11 +1171,7 @@ int run_waves(lux_ctx* C, int first_iter, int n_iter) {
         }
         int ns = std::min(spw, n_iter - w * spw);
         C->stats.samples += double(ns) * C->npix;
-        C->stats.launches_camera += 1;
-        C->stats.launches_accum += 1;
-        C->stats.launches_trace += depth * (nee ? 2 : 1);
-        C->stats.launches_shade += depth;
-        C->stats.launches_sort += C->opt.ray_sorting ? depth * sort_launches : 0;
+        count_launches(C, ns * C->npix);
         if (C->timing) {
             const cudaEvent_t* e = &C->kev[size_t(w) * epw];
             float t;
@@ -1416,6 +1457,7 @@ int ctx_finish(lux_ctx* C) {
     // occupancy queries happen here, never inside a stream capture
     for (int m = 0; m < 4; ++m) trace_grid_blocks(m, C->S.single_level != 0);
     shade_grid_blocks();
+    path_grid_blocks();
     if (cudaStreamSynchronize(C->stream) != cudaSuccess) return fail(LUX_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
     if (cudaGetLastError() != cudaSuccess) return fail(LUX_ERR_CUDA, "context set-up failed");
     return LUX_OK;

@@ -121,6 +121,9 @@ struct DevOptions {
 //   count[b]     queue length entering bounce b (count[0] = paths of the wave)
 //   shadow[b]    shadow rays queued at bounce b
 //   fetch_r[b], fetch_s[b]  work-fetch cursors of the persistent trace kernels
+//   fetch_p      work-fetch cursor of the whole-path kernel
+//   finished     bounce + 1 from which the whole-path kernel finished the lane's paths (0: it has
+//                not): the wavefront launches of later bounces then find no work
 //   error        sticky error word (bit 0: traversal stack overflow, bit 1: a wait of the ray
 //                sort gave up)
 constexpr int kMaxDepth = 64;
@@ -130,7 +133,9 @@ struct WaveCounters {
     int fetch_r[kMaxDepth];
     int fetch_s[kMaxDepth];
     int error;
-    int pad[3];
+    int fetch_p;
+    int finished;
+    int pad[1];
 };
 
 // One render job of the shared wavefront (job engine): a scene, a camera and resolution, a

@@ -10,6 +10,8 @@ constexpr int kTraceBlock = 128;
 constexpr int kShadeBlock = 384;  // three blocks per SM; both measured, see k_shade
 constexpr int kShadeOcc = 3;
 constexpr int kCameraBlock = 128;
+constexpr int kPathBlock = 128;  // three blocks per SM; see k_paths
+constexpr int kPathOcc = 3;
 
 // persistent traversal grid of `mode` for the two-level or the single-level layout
 int trace_grid_blocks(int mode, bool single = false);
@@ -41,6 +43,12 @@ size_t trace_static_scratch_bytes();
 // identity; wave_iter: the wave's first iteration and sample count (device)
 cudaError_t launch_camera(const DevScene& S, const DevWave& W, const DevOptions& O, const DevCamera& cam, int n,
                           int lane, const int* wave_iter, cudaStream_t st);
+// the paths of the segments to their end (`depth` bounces; job engine: each job's trace depth) in
+// one launch, paths.cu. It does nothing when they are more than `limit`; when it does run, later
+// wavefront launches of those lanes find them finished.
+cudaError_t launch_paths(const DevScene& S, const DevWave& W, const DevOptions& O, const Segs& G, int depth, int limit,
+                         cudaStream_t st);
+int path_grid_blocks();
 // shade bounce `bounce` (depth = bounce + 1 after the increment of src/pathtrace.cu:264)
 cudaError_t launch_shade(const DevScene& S, const DevWave& W, const DevOptions& O, int bounce, int compact,
                          cudaStream_t st);
@@ -64,6 +72,7 @@ cudaError_t launch_convert_texels(const void* src, int fmt, int to_half, void* d
 cudaError_t launch_morton_sort(const DevScene& S, DevWave& W, int bounce, void* temp, size_t temp_bytes,
                                cudaStream_t st);
 size_t morton_sort_temp_bytes(int max_paths);
+constexpr int kSortLaunches = 5;  // of one launch_morton_sort
 // before the first bounce of a wave: the sort's counters start at zero
 cudaError_t clear_sort_counters(void* temp, cudaStream_t st);
 cudaError_t launch_morton_ext(const DevScene& S, const float* rays, uint32_t* keys, int n, cudaStream_t st);
