@@ -65,6 +65,9 @@ struct PathArgs {
 template <bool JOBS, int NEE, bool SINGLE>
 __global__ void __launch_bounds__(kPathBlock, kPathOcc) k_paths(const __grid_constant__ PathArgs A) {
     __shared__ uint2 stack[kShStack][kPathBlock];
+    __shared__ float4 hits[kPathBlock];
+    __shared__ unsigned char lut[2048];
+    fill_key_table(lut);  // read after the barrier below
     __shared__ int seg_first[kMaxSegs + 1];
     // this block's share of the counters: survivors entering each bounce and shadow rays
     __shared__ int n_path[kMaxSegs][kMaxDepth + 1], n_shadow[kMaxSegs][kMaxDepth];
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(kPathBlock, kPathOcc) k_paths(const __grid_con
         bool hit = false;
 #pragma unroll 1
         for (int k = 0; k < (NEE ? 2 : 1); ++k) {
-            Tracer<NEE == 2 ? -1 : 0, SINGLE, PathKey> T{A.S, stack, {}, int(threadIdx.x), err, PathKey{p}, k == 1};
+            Tracer<NEE == 2 ? -1 : 0, SINGLE, PathKey> T{A.S, stack, hits, lut, {}, int(threadIdx.x), err, PathKey{p}, k == 1};
             Lane L;
             bool active = has;
             if (k == 0) {
@@ -177,10 +180,10 @@ __global__ void __launch_bounds__(kPathBlock, kPathOcc) k_paths(const __grid_con
             while (__any_sync(FULL, active))
                 if (T.step(L, active, postpone)) active = false;
             if (on && k == 0) {
-                best = L.best;
+                best = T.best(L);
                 hit = best.inst >= 0;
             } else if (on) {
-                sh = L.best;
+                sh = T.best(L);
             }
         }
         if (NEE == 2 && hit) sh.t = sh.inst >= 0 ? 1.0f : -1.0f;

@@ -48,27 +48,51 @@ struct TraceArgs {
 };
 
 
-// The key of a ray's alpha-blend hash: of wave rays the path id (pixel in s2.w, iteration in
-// s3.w), of rays given directly the pixel.
+// The segment of a slot: the one that holds the slot's lane.
+LUX_DI int seg_of_slot(const TraceArgs& A, int slot) {
+    int k = 0;
+    if (A.G.n > 1) {
+        const int ln = slot / A.W.lane_stride;
+        while (k + 1 < A.G.n && A.G.lane[k] != ln) ++k;
+    }
+    return k;
+}
+
+// The key of a ray's alpha-blend hash: of wave rays (item: the radiance ray's slot) the path's
+// pixel and iteration, of rays given directly the pixel that came with the ray.
 struct WaveKey {
     const TraceArgs& A;  // the launch's arguments, in parameter space like the scene
-    LUX_DI void operator()(int key, int& pixel, int& iter) const {
-        pixel = key;
-        iter = A.ext_iter;
-        if (A.ext_rays == nullptr) {
-            pixel = __float_as_int(A.W.s2[key].w);
-            iter = __float_as_int(A.W.s3[key].w);
+    LUX_DI void operator()(int item, int& pixel, int& iter) const {
+        if (A.ext_rays) {
+            pixel = __float_as_int(A.ext_rays[size_t(item) * 8 + 7]);
+            iter = A.ext_iter;
+            return;
         }
+        const int pid = A.W.queue[A.G.bounce[seg_of_slot(A, item)] & 1][item];
+        pixel = __float_as_int(A.W.s2[pid].w);
+        iter = __float_as_int(A.W.s3[pid].w);
     }
 };
 
 template <int MODE, bool SINGLE>
 // The arguments stay in parameter space (__grid_constant__): the tracer reads the scene
 // through a reference to them, which would otherwise copy the struct to local memory.
-// Seven 128-thread blocks per SM (at most 73 registers) measured faster than six (80) and
-// eight (64, with spills).
+// Seven 128-thread blocks per SM (72 registers) measured faster than six (80) and eight (64, with
+// spills): 32.9, 35.1 and 35.1 ms of traversal per 16-spp step of the 1M-triangle 1080p scene.
+// The loop is bound by instruction issue and the latency of dependent loads (bounce 1 of that
+// scene: 64 % issue, ALU pipe 54 %, L1 hit 61 %, 3.4 of 10.5 stall cycles on loads), so what counts
+// is instructions: 324 per thread and ray after the following, 421 before. Traversal per step:
+// 36.4 ms; 35.7 with the closest hit in shared memory, one limit register and the sign-bit slab
+// test; 33.9 with the plane distances two to an instruction (fma.rn.f32x2, which lost before the
+// registers were freed); 32.9 without the two-level layout's marker test in the single-level pop;
+// 32.7 with the key order from a table; 32.2 without its instance phase. Tried on top: the node's
+// own constants two to an instruction (35.1, spills), plane bytes by dp4a instead of byte permutes
+// (32.2), prefetching the next node before the triangle tests (33.1).
 __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant__ TraceArgs A) {
     __shared__ uint2 stack[kShStack][kTraceBlock];
+    __shared__ float4 hits[kTraceBlock];
+    __shared__ unsigned char lut[2048];
+    fill_key_table(lut);  // read after the barrier below
     // work of segment k: items [seg_first[k], seg_first[k + 1]) of the launch's list
     __shared__ int seg_first[kMaxSegs + 1];
     const bool ext = A.ext_rays != nullptr;
@@ -86,7 +110,7 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
         }
     }
     __syncthreads();
-    Tracer<MODE, SINGLE, WaveKey> T{A.S, stack, {}, int(threadIdx.x), &(A.W.ctr + A.G.lane[0])->error, WaveKey{A}, MODE == 2};
+    Tracer<MODE, SINGLE, WaveKey> T{A.S, stack, hits, lut, {}, int(threadIdx.x), &(A.W.ctr + A.G.lane[0])->error, WaveKey{A}, MODE == 2};
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int total;
@@ -107,49 +131,46 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
     bool active = false;
     bool exhausted = false;  // warp-uniform: the cursor has passed the end of the work list
     bool pending = false;    // the lane's ray is done and its result not yet written
-    int item = 0;
+    L.item = 0;
     while (true) {
         // Results of the rays that finished, written by all such lanes of the warp together
         // (at least 32 - kRefill of them, or the last ones): a lane that finishes keeps its
         // ray state untouched until the refill below replaces it.
         if (pending) {
             pending = false;
+            const Best best = T.best(L);
+            const int item = L.item;
             if (ext) {
                 uint32_t* h = A.ext_hits + size_t(item) * 5;
                 if (MODE == 2) {
-                    h[0] = __float_as_uint(L.best.inst >= 0 ? 1.0f : -1.0f);
+                    h[0] = __float_as_uint(best.inst >= 0 ? 1.0f : -1.0f);
                     h[1] = h[2] = 0xffffffffu;
                     h[3] = h[4] = 0u;
                 } else if (MODE == 3) {
-                    h[0] = __float_as_uint(L.best.inst >= 0 ? L.best.t : -1.0f);
-                    h[1] = uint32_t(L.best.inst);
-                    h[2] = uint32_t(L.best.prim);
+                    h[0] = __float_as_uint(best.t);
+                    h[1] = uint32_t(best.inst);
+                    h[2] = uint32_t(best.prim);
                     h[3] = uint32_t(L.work);
                     h[4] = 0u;
                 } else {
-                    h[0] = __float_as_uint(L.best.inst >= 0 ? L.best.t : -1.0f);
-                    h[1] = uint32_t(L.best.inst);
-                    h[2] = uint32_t(L.best.prim);
-                    h[3] = __float_as_uint(L.best.inst >= 0 ? L.best.u : 0.0f);
-                    h[4] = __float_as_uint(L.best.inst >= 0 ? L.best.v : 0.0f);
+                    h[0] = __float_as_uint(best.t);
+                    h[1] = uint32_t(best.inst);
+                    h[2] = uint32_t(best.prim);
+                    h[3] = __float_as_uint(best.u);
+                    h[4] = __float_as_uint(best.v);
                 }
             } else if (MODE == 0) {
-                bool hit = L.best.inst >= 0;
-                st_stream(&A.W.hit[item], make_float4(hit ? L.best.t : -1.0f, L.best.u, L.best.v, __int_as_float(L.best.inst)));
-                st_stream(&A.W.hit_prim[item], L.best.prim);
+                bool hit = best.inst >= 0;
+                st_stream(&A.W.hit[item], make_float4(best.t, best.u, best.v, __int_as_float(best.inst)));
+                st_stream(&A.W.hit_prim[item], best.prim);
                 if (hit && A.nee) {
-                    // the segment of this slot: its lane, then the segment holding that lane
-                    int k = 0;
-                    if (A.G.n > 1) {
-                        const int ln = item / A.W.lane_stride;
-                        while (k + 1 < A.G.n && A.G.lane[k] != ln) ++k;
-                    }
+                    const int k = seg_of_slot(A, item);
                     const int bk = A.G.bounce[k], lk = A.G.lane[k];
                     int pid = ld_stream(&A.W.queue[bk & 1][item]);
                     float4 ns = ld_stream(&A.W.s4[pid]);
                     f3 so, sd;
                     float tmax;
-                    shadow_ray(A.S, L.best, T.world_o(L), T.world_d(L), mk(ns.x, ns.y, ns.z), A.nee == 2, so, sd, tmax);
+                    shadow_ray(A.S, best, T.world_o(L), T.world_d(L), mk(ns.x, ns.y, ns.z), A.nee == 2, so, sd, tmax);
                     // append to the lane's shadow queue, aggregated over the lanes of the
                     // warp that append to the same one; the ray is stored at its queue
                     // position, beside the slot it belongs to, so the occlusion launch reads
@@ -165,9 +186,9 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
                     st_stream(&A.W.sh_queue[q], item);
                 }
             } else if (MODE == 1) {
-                bool hit = L.best.inst >= 0;
-                st_stream(&A.W.sh_hit[item], make_float4(hit ? L.best.t : -1.0f, L.best.u, L.best.v, __int_as_float(L.best.inst)));
-                st_stream(&A.W.sh_prim[item], L.best.prim);
+                bool hit = best.inst >= 0;
+                st_stream(&A.W.sh_hit[item], make_float4(best.t, best.u, best.v, __int_as_float(best.inst)));
+                st_stream(&A.W.sh_prim[item], best.prim);
             } else if (MODE == 3) {
                 // drawBVH (src/kernels/draw_bvh.cu:33): color += count * 0.001 on every channel
                 int pid = A.W.queue[A.G.bounce[0] & 1][item];  // the heatmap traces one wave
@@ -175,7 +196,7 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
                 const float h = float(L.work) * 0.001f;
                 A.W.s3[pid] = make_float4(c.x + h, c.y + h, c.z + h, c.w);
             } else {
-                st_stream(&A.W.sh_hit[item], make_float4(L.best.inst >= 0 ? 1.0f : -1.0f, 0.0f, 0.0f, __int_as_float(-1)));
+                st_stream(&A.W.sh_hit[item], make_float4(best.inst >= 0 ? 1.0f : -1.0f, 0.0f, 0.0f, __int_as_float(-1)));
             }
         }
         unsigned need = __ballot_sync(FULL, !active);
@@ -187,17 +208,15 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
             if (!active) {
                 int r = base + __popc(need & ((1u << lane) - 1u));
                 if (r < total) {
-                    item = r;
+                    int item = r;
                     f3 o, d;
                     float tmax;
                     uint32_t root = A.S.tlas_root;
-                    L.key = 0;
                     if (ext) {
                         const float* ry = A.ext_rays + size_t(r) * 8;
                         o = mk(ry[0], ry[1], ry[2]);
                         d = mk(ry[4], ry[5], ry[6]);
                         tmax = MODE == 1 ? ry[3] : 1e16f;
-                        L.key = __float_as_int(ry[7]);
                     } else if (MODE == 0 || MODE == 3) {
                         int k = 0;
                         while (k + 1 < A.G.n && r >= seg_first[k + 1]) ++k;
@@ -207,7 +226,6 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
                         o = mk(a.x, a.y, a.z);
                         d = mk(b.x, b.y, b.z);
                         tmax = 1e16f;
-                        L.key = pid;
                         if (A.W.path_job) root = A.W.jobs[A.W.path_job[pid]].tlas_root;
                     } else {
                         int k = 0;
@@ -220,9 +238,9 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
                         d = mk(b.x, b.y, b.z);
                         tmax = a.w;
                         int pid = ld_stream(&A.W.queue[A.G.bounce[k] & 1][slot]);
-                        L.key = pid;
                         if (A.W.path_job) root = A.W.jobs[A.W.path_job[pid]].tlas_root;
                     }
+                    L.item = item;
                     T.start(L, o, d, tmax, root);
                     active = true;
                 }

@@ -12,8 +12,9 @@
 namespace lux {
 namespace {
 
-constexpr int kShStack = 16;
-constexpr int kLocStack = 48;
+// stack entries in shared memory; 6 to 16 measured alike (the rest of a deep stack is in local memory)
+constexpr int kShStack = 12;
+constexpr int kLocStack = 52;
 static_assert(kShStack + kLocStack == kTraversalStack, "the scene build bounds the stack by kTraversalStack");
 constexpr int kRefill = 20;
 // environment occlusion rays (any hit, mode 2) refill below this many traversing lanes
@@ -32,6 +33,9 @@ constexpr int kPostpone = 6;
 // Slab acceptance tnear <= tfar * kWiden (tnear >= 0): a relative margin of 2^-17, far above
 // the few-ulp rounding of the plane distances.
 constexpr float kWiden = 1.0f + 1.0f / 131072.0f;
+// Boxes that end behind the origin are skipped; the bound lies a hair below 0, so that a far plane
+// at -0 still counts as at the origin when the sign bit of tf * kWiden - tn decides.
+constexpr float kBehind = -1e-30f;
 static_assert(kMaxLeafPrims == 1, "visit_node marks one triangle per leaf slot");
 
 struct TRay {
@@ -84,12 +88,46 @@ LUX_DI float min3f(float a, float b, float c) {
     return r;
 }
 
+LUX_DI unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+// Distances of planes b and b + 1 of word w: two lanes of one fma (sm_100), each rounded as fmaf.
+LUX_DI float2 planes(uint32_t w, int b, unsigned long long a, unsigned long long c) {
+    unsigned long long q = pack2(ubyte_biased(w, b), ubyte_biased(w, b + 1)), r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(q), "l"(a), "l"(c));
+    float2 o;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(o.x), "=f"(o.y) : "l"(r));
+    return o;
+}
+
+// missed << 1 | whether the slab test misses. The sign of tf * kWiden - tn decides, one multiply-add
+// and a funnel shift for a multiply, a compare and a bit.
+LUX_DI uint32_t miss_bit(uint32_t missed, float tnx, float tny, float tnz, float tfx, float tfy, float tfz, float tmax) {
+    const float tn = max3f(tnx, tny, fmaxf(tnz, kBehind));
+    const float tf = min3f(tfx, tfy, fminf(tfz, tmax));
+    return __funnelshift_l(__float_as_uint(fmaf(tf, kWiden, -tn)), missed, 1);
+}
+
+// Table of the slot masks in key order: bit s of lut[oct << 8 | mask] is bit s ^ oct of mask.
+LUX_DI void fill_key_table(unsigned char* lut) {
+    for (int i = threadIdx.x; i < 2048; i += blockDim.x) {
+        uint32_t m = i & 255;
+        const int oct = i >> 8;
+        if (oct & 1) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
+        if (oct & 2) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
+        if (oct & 4) m = ((m & 0x0Fu) << 4) | ((m >> 4) & 0x0Fu);
+        lut[i] = (unsigned char)m;
+    }
+}
+
 // Intersect the 8 child boxes of node ni. Returns internal-child hits as a key mask
 // (bit slot ^ oct), leaf hits as a slot mask, the node's leaf-slot mask, child_base and
 // tri_base.
 LUX_DI void visit_node(const uint4* __restrict__ nodes, uint32_t ni, const TRay& r, float tmax, uint32_t& keys,
                        uint32_t& imask, uint32_t& child_base, uint32_t& tri_base, uint32_t& trimask,
-                       uint32_t& leafmask) {
+                       uint32_t& leafmask, const unsigned char* lut) {
     const uint4* n = nodes + size_t(ni) * 5;
     uint4 w0 = __ldg(n + 0), w1 = __ldg(n + 1), w2 = __ldg(n + 2), w3 = __ldg(n + 3), w4 = __ldg(n + 4);
     float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
@@ -113,41 +151,31 @@ LUX_DI void visit_node(const uint4* __restrict__ nodes, uint32_t ni, const TRay&
     uint32_t nx0 = fx ? w3.z : w2.x, nx1 = fx ? w3.w : w2.y, fx0 = fx ? w2.x : w3.z, fx1 = fx ? w2.y : w3.w;
     uint32_t ny0 = fy ? w4.x : w2.z, ny1 = fy ? w4.y : w2.w, fy0 = fy ? w2.z : w4.x, fy1 = fy ? w2.w : w4.y;
     uint32_t nz0 = fz ? w4.z : w3.x, nz1 = fz ? w4.w : w3.y, fz0 = fz ? w3.x : w4.z, fz1 = fz ? w3.y : w4.w;
-    uint32_t hits = 0;
+    uint32_t missed = 0;
+    const unsigned long long ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
+    const unsigned long long bx2 = pack2(bx, bx), by2 = pack2(by, by), bz2 = pack2(bz, bz);
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
+    for (int s = 6; s >= 0; s -= 2) {
         const int b = s & 3;
         uint32_t wnx = s < 4 ? nx0 : nx1, wny = s < 4 ? ny0 : ny1, wnz = s < 4 ? nz0 : nz1;
         uint32_t wfx = s < 4 ? fx0 : fx1, wfy = s < 4 ? fy0 : fy1, wfz = s < 4 ? fz0 : fz1;
-        float tnx = fmaf(ubyte_biased(wnx, b), ax, bx), tny = fmaf(ubyte_biased(wny, b), ay, by),
-              tnz = fmaf(ubyte_biased(wnz, b), az, bz);
-        float tfx = fmaf(ubyte_biased(wfx, b), ax, bx), tfy = fmaf(ubyte_biased(wfy, b), ay, by),
-              tfz = fmaf(ubyte_biased(wfz, b), az, bz);
-        float tn = max3f(tnx, tny, fmaxf(tnz, 0.0f));
-        float tf = min3f(tfx, tfy, fminf(tfz, tmax));
-        if (tn <= tf * kWiden) hits |= 1u << s;
+        float2 tnx = planes(wnx, b, ax2, bx2), tny = planes(wny, b, ay2, by2), tnz = planes(wnz, b, az2, bz2);
+        float2 tfx = planes(wfx, b, ax2, bx2), tfy = planes(wfy, b, ay2, by2), tfz = planes(wfz, b, az2, bz2);
+        missed = miss_bit(missed, tnx.y, tny.y, tnz.y, tfx.y, tfy.y, tfz.y, tmax);
+        missed = miss_bit(missed, tnx.x, tny.x, tnz.x, tfx.x, tfy.x, tfz.x, tmax);
     }
     leafmask = w1.z & 0xffu;
-    hits &= imask | leafmask;
+    const uint32_t hits = ~missed & (imask | leafmask);
     trimask = hits & leafmask;
-    uint32_t ih = hits & imask;  // to key order: bit s moves to bit s ^ oct
-    if (r.oct & 1) ih = ((ih & 0x55u) << 1) | ((ih >> 1) & 0x55u);
-    if (r.oct & 2) ih = ((ih & 0x33u) << 2) | ((ih >> 2) & 0x33u);
-    if (r.oct & 4) ih = ((ih & 0x0Fu) << 4) | ((ih >> 4) & 0x0Fu);
-    keys = ih;
+    keys = lut[(r.oct << 8) | (hits & imask)];
 }
 
+// A ray's closest hit; inst -1: none.
 struct Best {
     float t;
     int inst, prim;
     float u, v;
 };
-
-LUX_DI bool better(float t, int inst, int prim, const Best& b) {
-    if (b.inst < 0) return true;
-    if (t < b.t) return true;
-    return t == b.t && (inst < b.inst || (inst == b.inst && prim < b.prim));
-}
 
 // Moller-Trumbore exactly as src/intersections/mesh_isect.cu:78-115, single-rounded ops, on a
 // triangle record (v0 with the triangle index in w, e1, e2) and the ray (ro, d) of the
@@ -228,8 +256,7 @@ LUX_DI bool alpha_accept(const DevScene& S, const DevInstance& I, int inst, int 
 struct Lane {
     f3 wo, wd;          // world ray (two-level) / object ray of `inst` (single-level)
     TRay cur;           // ray of the current level (world in the TLAS, object space in a BLAS)
-    float tmax;
-    Best best;
+    float tlim;         // the ray's limit: tmax until a hit, then the closest hit's t
     uint2 g;            // node group: x = first internal child, y = imask << 8 | remaining hit keys
     uint2 t;            // leaf group: x = first record, y = tag (kTagTri / kTagInst) | leaf-slot
                         // mask << 8 | remaining hit slots
@@ -237,8 +264,8 @@ struct Lane {
     int inst;           // current instance (-1 in the TLAS)
     int inst_flags;
     uint32_t inst_prim_base;
-    int key;            // path id (wave rays) or pixel (rays given directly): the alpha-blend
-                        // hash key, resolved only when an alpha-blended instance is tested
+    int item;           // the ray's work item, from which the alpha-blend hash key is found when an
+                        // alpha-blended instance is tested
     int work;           // BVH heatmap (mode 3): node visits + triangle tests
     bool done;
 };
@@ -250,6 +277,8 @@ template <int MODE, bool SINGLE, class KEY>
 struct Tracer {
     const DevScene& S;
     uint2 (*sh)[kTraceBlock];  // shared stack [kShStack][block]
+    float4* hits;              // shared, per thread: the closest hit's u, v, instance, prim (int bits)
+    const unsigned char* lut;  // shared, fill_key_table
     uint2 loc[kLocStack];
     int tid;
     int* err;
@@ -276,11 +305,8 @@ struct Tracer {
         L.wo = o;
         L.wd = d;
         L.cur = make_ray(o, d);
-        L.tmax = tmax;
-        L.best.t = -1.0f;
-        L.best.inst = -1;
-        L.best.prim = -1;
-        L.best.u = L.best.v = 0.0f;
+        L.tlim = tmax;
+        hits[tid] = make_float4(0.0f, 0.0f, __int_as_float(-1), __int_as_float(-1));
         L.sp = 0;
         L.inst = -1;
         L.inst_flags = 0;
@@ -292,7 +318,16 @@ struct Tracer {
         L.t = make_uint2(0u, 0u);
     }
 
-    LUX_DI float limit(const Lane& L) const { return (!any_hit() && L.best.inst >= 0) ? L.best.t : L.tmax; }
+    LUX_DI Best best(const Lane& L) const {
+        const float4 h = hits[tid];
+        Best b;
+        b.u = h.x;
+        b.v = h.y;
+        b.inst = __float_as_int(h.z);
+        b.prim = __float_as_int(h.w);
+        b.t = b.inst >= 0 ? L.tlim : -1.0f;
+        return b;
+    }
     static LUX_DI f3 world_o(const Lane& L) { return SINGLE ? L.cur.o : L.wo; }
     static LUX_DI f3 world_d(const Lane& L) { return SINGLE ? L.cur.d : L.wd; }
 
@@ -306,7 +341,7 @@ struct Tracer {
         uint32_t child = L.g.x + __popc(imask & ((1u << slot) - 1u));
         if (keys) push(L, make_uint2(L.g.x, (imask << 8) | keys));
         uint32_t nkeys, nimask, cbase, tbase, tmask, lmask;
-        visit_node(S.nodes, child, L.cur, limit(L), nkeys, nimask, cbase, tbase, tmask, lmask);
+        visit_node(S.nodes, child, L.cur, L.tlim, nkeys, nimask, cbase, tbase, tmask, lmask, lut);
         if (MODE == 3) ++L.work;
         L.g = make_uint2(cbase, (nimask << 8) | nkeys);
         if (tmask) {
@@ -347,18 +382,19 @@ struct Tracer {
         } else {
             if (!mt_test(S.prims, L.t.x + uint32_t(k), L.cur, t, u, v, prim)) return;
         }
-        if (!(t <= L.tmax)) return;
-        if (!any_hit() && !better(t, L.inst, prim, L.best)) return;
+        if (!(t <= L.tlim)) return;
+        if (!any_hit() && t == L.tlim) {  // a tie with a hit goes to the lowest (instance, prim)
+            const float4 h = hits[tid];
+            const int bi = __float_as_int(h.z), bp = __float_as_int(h.w);
+            if (bi >= 0 && !(L.inst < bi || (L.inst == bi && prim < bp))) return;
+        }
         if (L.inst_flags & kInstAnyHit) {
             int pixel, iter;
-            keys(L.key, pixel, iter);
+            keys(L.item, pixel, iter);
             if (!alpha_accept(S, S.insts[L.inst], L.inst, prim, u, v, world_d(L), pixel, iter)) return;
         }
-        L.best.t = t;
-        L.best.inst = L.inst;
-        L.best.prim = prim;
-        L.best.u = u;
-        L.best.v = v;
+        L.tlim = t;
+        hits[tid] = make_float4(u, v, __int_as_float(L.inst), __int_as_float(prim));
         if (any_hit()) L.done = true;
     }
 
@@ -396,7 +432,7 @@ struct Tracer {
             }
             uint2 e = pop(L);
             uint32_t tag = e.y & kTagMask;
-            if (tag == kTagMarker) {
+            if (!SINGLE && tag == kTagMarker) {
                 L.cur = make_ray(L.wo, L.wd);
                 L.inst = -1;
                 L.inst_flags = 0;
@@ -417,7 +453,7 @@ struct Tracer {
         if (active && (L.g.y & 0xffu)) visit(L);
         // triangle phase, postponed while too few lanes have triangles and others nodes
         while (true) {
-            const bool want = active && (L.t.y & kTagMask) == kTagTri;
+            const bool want = active && (SINGLE ? L.t.y != 0u : (L.t.y & kTagMask) == kTagTri);
             const unsigned wm = __ballot_sync(FULL, want);
             if (!wm) break;
             const bool nodes = active && (L.g.y & 0xffu);
@@ -436,7 +472,7 @@ struct Tracer {
             }
         }
         // instance phase
-        if (active && !L.done && (L.t.y & kTagMask) == kTagInst) enter(L);
+        if (!SINGLE && active && !L.done && (L.t.y & kTagMask) == kTagInst) enter(L);
         // pop phase
         if (active && !L.done && !(L.g.y & 0xffu) && !(L.t.y & kRecMask)) next(L);
         return active && L.done;
