@@ -317,17 +317,16 @@ int lux_trace_rays(lux_ctx* ctx, const float* rays, int n, int mode, int iter, u
  * lux_trace_rays, for n <= LUX_TRACE_STATIC_MAX_RAYS; a larger n is rejected with
  * LUX_ERR_INVALID before any device work.
  * Who needs it: a host that has given the device's free memory to its own pool or to other
- * tenants under a fixed budget, where a per-call cudaMalloc can fail in the middle of a
- * request; and a host that keeps other work running on other streams of the device, which
- * the per-call cudaFree of lux_trace_rays stalls (cudaFree waits for the whole device).
+ * tenants under a fixed budget, where lux_trace_rays' per-call allocation (stream-ordered, from
+ * the library's pool) can fail in the middle of a request.
  * Rays and hits are staged through one fixed array of 256 + 52 * LUX_TRACE_STATIC_MAX_RAYS
  * bytes (about 3.25 MiB) compiled into the library, one copy per device. Its address is
  * looked up (cudaGetSymbolAddress) on every call; the first call on a device may load the
  * library's device code there, so make that first call before any stream capture begins on
  * that device.
- * Must start at zero: the traversal's work cursor in that array and the context's traversal
- * error word; the call clears both on the context's stream before its launch. Nothing else
- * carries over from one call to the next.
+ * Must start at zero: the traversal's work cursor in that array, which the call clears on the
+ * context's stream before its launch, and its error word, which is in page-locked host memory of
+ * the call. Nothing else carries over from one call to the next.
  * Calls that overlap on one device (two threads, or two contexts on the same device) share
  * the array and race: the library does not lock it, so serialise such calls. */
 #define LUX_TRACE_STATIC_MAX_RAYS 65536

@@ -45,6 +45,7 @@ struct TraceArgs {
     int ext_n;
     int ext_iter;
     int* ext_fetch;
+    int* ext_err;           // and its error word, which the host can read (page-locked)
 };
 
 
@@ -60,10 +61,11 @@ LUX_DI int seg_of_slot(const TraceArgs& A, int slot) {
 
 // The key of a ray's alpha-blend hash: of wave rays (item: the radiance ray's slot) the path's
 // pixel and iteration, of rays given directly the pixel that came with the ray.
-struct WaveKey {
+template <bool EXT>
+struct RayKey {
     const TraceArgs& A;  // the launch's arguments, in parameter space like the scene
     LUX_DI void operator()(int item, int& pixel, int& iter) const {
-        if (A.ext_rays) {
+        if (EXT) {
             pixel = __float_as_int(A.ext_rays[size_t(item) * 8 + 7]);
             iter = A.ext_iter;
             return;
@@ -74,7 +76,12 @@ struct WaveKey {
     }
 };
 
-template <int MODE, bool SINGLE>
+// Rays given directly are spread over the warps up to this many per warp: 20,000 rays (5 a warp)
+// 251 -> 237 us a call, 100 rays 81 -> 68, but 65,536 rays (16 a warp) 438 -> 482.
+constexpr int kSpread = 8;
+
+// EXT: rays given directly (lux_trace_rays); else the rays of waves.
+template <int MODE, bool SINGLE, bool EXT>
 // The arguments stay in parameter space (__grid_constant__): the tracer reads the scene
 // through a reference to them, which would otherwise copy the struct to local memory.
 // Seven 128-thread blocks per SM (72 registers) measured faster than six (80) and eight (64, with
@@ -88,19 +95,18 @@ template <int MODE, bool SINGLE>
 // 32.7 with the key order from a table; 32.2 without its instance phase. Tried on top: the node's
 // own constants two to an instruction (35.1, spills), plane bytes by dp4a instead of byte permutes
 // (32.2), prefetching the next node before the triangle tests (33.1).
-__global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant__ TraceArgs A) {
+__global__ void __launch_bounds__(kTraceBlock, SINGLE ? 7 : 6) k_trace(const __grid_constant__ TraceArgs A) {
     __shared__ uint2 stack[kShStack][kTraceBlock];
     __shared__ float4 hits[kTraceBlock];
     __shared__ unsigned char lut[2048];
     fill_key_table(lut);  // read after the barrier below
     // work of segment k: items [seg_first[k], seg_first[k + 1]) of the launch's list
     __shared__ int seg_first[kMaxSegs + 1];
-    const bool ext = A.ext_rays != nullptr;
     if (threadIdx.x == 0) {
         int t = 0;
         seg_first[0] = 0;
         for (int k = 0; k < kMaxSegs; ++k) {
-            if (!ext && k < A.G.n) {
+            if (!EXT && k < A.G.n) {
                 const WaveCounters* c = A.W.ctr + A.G.lane[k];
                 if (*(volatile const int*)&c->finished == 0)
                     t += (MODE == 0 || MODE == 3) ? *(volatile const int*)&c->count[A.G.bounce[k]]
@@ -110,14 +116,15 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
         }
     }
     __syncthreads();
-    Tracer<MODE, SINGLE, WaveKey> T{A.S, stack, hits, lut, {}, int(threadIdx.x), &(A.W.ctr + A.G.lane[0])->error, WaveKey{A}, MODE == 2};
+    Tracer<MODE, SINGLE, RayKey<EXT>> T{A.S, stack, hits, lut, {}, int(threadIdx.x), EXT ? A.ext_err : &(A.W.ctr + A.G.lane[0])->error,
+                                        RayKey<EXT>{A}, MODE == 2};
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int total;
     int* cursor;
     // the cursor of the first segment's (lane, bounce) serves the whole launch: no other
     // launch of this kind covers that lane at that bounce
-    if (ext) {
+    if (EXT) {
         total = A.ext_n;
         cursor = A.ext_fetch;
     } else if (MODE == 0 || MODE == 3) {
@@ -127,6 +134,17 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
         total = seg_first[kMaxSegs];
         cursor = &(A.W.ctr + A.G.lane[0])->fetch_s[A.G.bounce[0]];
     }
+    // Rays given directly that are fewer than the grid's lanes are spread over all its warps: `cap`
+    // lanes of each take one, by the warp's place. A ray's time is its chain of dependent node
+    // visits, and rays of one warp wait for one another's phases; the postponement threshold shrinks
+    // with the warp's rays, or no triangle would be tested (and no limit shortened) before every
+    // lane had run out of nodes. (The waves' launches leave few rays to the whole-path kernel, and
+    // the two thresholds in registers cost their loop 1 to 2 %.)
+    const int warps = int(gridDim.x) * (kTraceBlock / 32);
+    int cap = 32;
+    if (EXT && total <= kSpread * warps) cap = (total + warps - 1) / warps;
+    const int postpone = EXT ? (cap * kPostpone) >> 5 : kPostpone;
+    const int refill = cap < 32 ? 0 : (MODE == 2 ? kRefillOcclusion : kRefill);
     Lane L;
     bool active = false;
     bool exhausted = false;  // warp-uniform: the cursor has passed the end of the work list
@@ -140,7 +158,7 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
             pending = false;
             const Best best = T.best(L);
             const int item = L.item;
-            if (ext) {
+            if (EXT) {
                 uint32_t* h = A.ext_hits + size_t(item) * 5;
                 if (MODE == 2) {
                     h[0] = __float_as_uint(best.inst >= 0 ? 1.0f : -1.0f);
@@ -199,20 +217,25 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
                 st_stream(&A.W.sh_hit[item], make_float4(best.inst >= 0 ? 1.0f : -1.0f, 0.0f, 0.0f, __int_as_float(-1)));
             }
         }
-        unsigned need = __ballot_sync(FULL, !active);
+        unsigned need = __ballot_sync(FULL, !active && lane < cap);
         if (need && !exhausted) {
             int base = 0;
-            if (lane == 0) base = atomicAdd(cursor, __popc(need));
-            base = __shfl_sync(FULL, base, 0);
-            if (base + __popc(need) >= total) exhausted = true;
-            if (!active) {
+            if (EXT && cap < 32) {  // blocks apart, so that a few rays reach many SMs
+                base = (int(threadIdx.x >> 5) * int(gridDim.x) + int(blockIdx.x)) * cap;
+                exhausted = true;
+            } else {
+                if (lane == 0) base = atomicAdd(cursor, __popc(need));
+                base = __shfl_sync(FULL, base, 0);
+                if (base + __popc(need) >= total) exhausted = true;
+            }
+            if (!active && lane < cap) {
                 int r = base + __popc(need & ((1u << lane) - 1u));
                 if (r < total) {
                     int item = r;
                     f3 o, d;
                     float tmax;
                     uint32_t root = A.S.tlas_root;
-                    if (ext) {
+                    if (EXT) {
                         const float* ry = A.ext_rays + size_t(r) * 8;
                         o = mk(ry[0], ry[1], ry[2]);
                         d = mk(ry[4], ry[5], ry[6]);
@@ -237,8 +260,10 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
                         o = mk(a.x, a.y, a.z);
                         d = mk(b.x, b.y, b.z);
                         tmax = a.w;
-                        int pid = ld_stream(&A.W.queue[A.G.bounce[k] & 1][slot]);
-                        if (A.W.path_job) root = A.W.jobs[A.W.path_job[pid]].tlas_root;
+                        if (A.W.path_job) {
+                            const int pid = ld_stream(&A.W.queue[A.G.bounce[k] & 1][slot]);
+                            root = A.W.jobs[A.W.path_job[pid]].tlas_root;
+                        }
                     }
                     L.item = item;
                     T.start(L, o, d, tmax, root);
@@ -248,15 +273,24 @@ __global__ void __launch_bounds__(kTraceBlock, 7) k_trace(const __grid_constant_
         }
         if (!__any_sync(FULL, active)) break;
         while (true) {
-            if (T.step(L, active, kPostpone)) {
+            if (T.step(L, active, postpone)) {
                 active = false;
                 pending = true;
             }
             const unsigned am = __ballot_sync(FULL, active);
             if (!am) break;
-            if (__popc(am) < (MODE == 2 ? kRefillOcclusion : kRefill) && !exhausted) break;
+            if (__popc(am) < refill && !exhausted) break;
         }
     }
+}
+
+// resident blocks per SM that both the waves' kernel and the direct rays' reach
+template <int MODE, bool SINGLE>
+int blocks_per_sm() {
+    int a = 0, b = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_trace<MODE, SINGLE, false>, kTraceBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace<MODE, SINGLE, true>, kTraceBlock, 0);
+    return a < b ? a : b;
 }
 
 }  // namespace
@@ -274,16 +308,15 @@ int trace_grid_blocks(int mode, bool single) {
     if (cached == 0) {
         int sms = 0, per = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (single) {
-            if (mode == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<0, true>, kTraceBlock, 0);
-            else if (mode == 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<1, true>, kTraceBlock, 0);
-            else if (mode == 2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<2, true>, kTraceBlock, 0);
-            else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<3, true>, kTraceBlock, 0);
-        } else {
-            if (mode == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<0, false>, kTraceBlock, 0);
-            else if (mode == 1) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<1, false>, kTraceBlock, 0);
-            else if (mode == 2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<2, false>, kTraceBlock, 0);
-            else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_trace<3, false>, kTraceBlock, 0);
+        switch (mode * 2 + (single ? 1 : 0)) {
+            case 0: per = blocks_per_sm<0, false>(); break;
+            case 1: per = blocks_per_sm<0, true>(); break;
+            case 2: per = blocks_per_sm<1, false>(); break;
+            case 3: per = blocks_per_sm<1, true>(); break;
+            case 4: per = blocks_per_sm<2, false>(); break;
+            case 5: per = blocks_per_sm<2, true>(); break;
+            case 6: per = blocks_per_sm<3, false>(); break;
+            default: per = blocks_per_sm<3, true>(); break;
         }
         cached = sms * (per > 0 ? per : 1);
     }
@@ -291,12 +324,12 @@ int trace_grid_blocks(int mode, bool single) {
 }
 
 namespace {
-template <bool SINGLE>
+template <bool SINGLE, bool EXT>
 void launch_mode(int mode, int grid, cudaStream_t st, const TraceArgs& A) {
-    if (mode == 0) k_trace<0, SINGLE><<<grid, kTraceBlock, 0, st>>>(A);
-    else if (mode == 1) k_trace<1, SINGLE><<<grid, kTraceBlock, 0, st>>>(A);
-    else if (mode == 2) k_trace<2, SINGLE><<<grid, kTraceBlock, 0, st>>>(A);
-    else k_trace<3, SINGLE><<<grid, kTraceBlock, 0, st>>>(A);
+    if (mode == 0) k_trace<0, SINGLE, EXT><<<grid, kTraceBlock, 0, st>>>(A);
+    else if (mode == 1) k_trace<1, SINGLE, EXT><<<grid, kTraceBlock, 0, st>>>(A);
+    else if (mode == 2) k_trace<2, SINGLE, EXT><<<grid, kTraceBlock, 0, st>>>(A);
+    else k_trace<3, SINGLE, EXT><<<grid, kTraceBlock, 0, st>>>(A);
 }
 }  // namespace
 
@@ -308,21 +341,21 @@ cudaError_t launch_trace(const DevScene& S, const DevWave& W, int bounce, int mo
 cudaError_t launch_trace_segs(const DevScene& S, const DevWave& W, const Segs& G, int mode, int nee, cudaStream_t st,
                               int grid) {
     if (G.n < 1 || G.n > kMaxSegs) return cudaErrorInvalidValue;
-    TraceArgs A{S, W, G, mode, nee, nullptr, nullptr, 0, 0, nullptr};
+    TraceArgs A{S, W, G, mode, nee, nullptr, nullptr, 0, 0, nullptr, nullptr};
     const bool single = S.single_level != 0;
     if (grid <= 0) grid = trace_grid_blocks(mode, single);
-    if (single) launch_mode<true>(mode, grid, st, A);
-    else launch_mode<false>(mode, grid, st, A);
+    if (single) launch_mode<true, false>(mode, grid, st, A);
+    else launch_mode<false, false>(mode, grid, st, A);
     return cudaGetLastError();
 }
 
 cudaError_t launch_trace_ext(const DevScene& S, const DevWave& W, const float* rays, uint32_t* hits, int n, int mode,
-                             int iter, int* fetch, cudaStream_t st) {
-    TraceArgs A{S, W, one_seg(0), mode, 0, rays, hits, n, iter, fetch};
+                             int iter, int* fetch, int* err, cudaStream_t st) {
+    TraceArgs A{S, W, one_seg(0), mode, 0, rays, hits, n, iter, fetch, err};
     const bool single = S.single_level != 0;
     const int grid = trace_grid_blocks(mode, single);
-    if (single) launch_mode<true>(mode, grid, st, A);
-    else launch_mode<false>(mode, grid, st, A);
+    if (single) launch_mode<true, true>(mode, grid, st, A);
+    else launch_mode<false, true>(mode, grid, st, A);
     return cudaGetLastError();
 }
 

@@ -1,7 +1,7 @@
 // trace_static.cu -- the fixed device scratch behind lux_trace_rays_static.
 //
-// lux_trace_rays stages a batch of caller rays through three per-call cudaMalloc temporaries
-// (rays, hits, the work cursor of the persistent traversal). lux_trace_rays_static stages them
+// lux_trace_rays stages a batch of caller rays through a per-call block of the library's memory
+// pool (rays, hits, the work cursor of the persistent traversal). lux_trace_rays_static stages them
 // through this one array instead, compiled into the library, so the call allocates nothing.
 // Each device holds its own copy of the array; its address is looked up with
 // cudaGetSymbolAddress on every call, with that device current, so a device reset (which
