@@ -1,19 +1,22 @@
 // bvh_gpu.cu -- device build of the compressed 8-wide BVH (bvh_gpu.h).
 //
 // Binary stage (binned SAH, one primitive per leaf), over all trees at once:
-//   * nodes of more than kSmall primitives are split level by level: their ranges are cut into
+//   * nodes of more than kMedium primitives are split level by level: their ranges are cut into
 //     chunks of kChunk primitives, one block per chunk; a pass reduces each node's box and
 //     centroid bounds, a pass bins the centroids (32 bins per live axis, shared-memory bins
 //     merged into the node's bins with atomic min/max on order-preserving integer keys), one
 //     thread per node sweeps the bins in double, and a stable two-pass scatter partitions the
 //     node's range;
+//   * a node of kSmall + 1 .. kMedium primitives is handed to one block, which splits it and its
+//     descendants down to kSmall primitives in shared memory;
 //   * a node of 2..kSmall primitives is handed to one warp, which builds its whole subtree with
 //     one primitive per lane, shuffles for the reductions and the sweep, and a ballot for the
 //     stable partition.
-// Collapse stage, level by level over the 8-wide levels of all trees at once: one thread per
-// 8-wide node opens the child of largest area until 8 slots are filled, assigns slots by child
-// centroid octant and quantises the child boxes; exclusive scans give every node's children
-// and leaf records their places, breadth first within its tree, trees one after another.
+// Collapse stage, level by level over the 8-wide levels of all trees at once: eight lanes per
+// 8-wide node open the child of largest area until 8 slots are filled, assign slots by child
+// centroid octant and quantise the child boxes; a look-back over the level's tiles gives every
+// node's children and leaf records their places, breadth first within its tree, trees one after
+// another.
 // Every floating-point step is the host builder's (bvh_build.cpp), rounded the same way, and
 // every tie is broken the same way, so the nodes are identical to the host build's.
 
@@ -22,6 +25,7 @@
 
 #include <cfloat>
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <mutex>
 
@@ -70,6 +74,7 @@ namespace {
 
 constexpr int kBins = 32;
 constexpr int kSmall = 32;      // nodes of at most this many primitives: one warp per subtree
+constexpr int kMedium = 1024;   // nodes of at most this many: one block down to kSmall
 constexpr int kChunk = 2048;    // primitives per block in the large-node passes
 constexpr int kBlock = 256;
 constexpr int kPerThread = kChunk / kBlock;
@@ -123,10 +128,10 @@ __device__ __forceinline__ int ceil_log2(double x) {
 // binary stage: set-up
 // ---------------------------------------------------------------------------------------------
 
-// Roots: node t is tree t's root; identity order; lists of large and small roots; single-
+// Roots: node t is tree t's root; identity order; lists of large, medium and small roots; single-
 // primitive trees are leaves at once.
 __global__ void k_roots(const float* boxes, const int* tree_begin, int num_trees, BinNode* bn, int* ord0, int* ord_fin,
-                        int* large, int* n_large, int* small, int* n_small) {
+                        int* large, int* n_large, unsigned* medium, int* n_medium, int* small, int* n_small) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < num_trees; t += gridDim.x * blockDim.x) {
         const int b = tree_begin[t], n = tree_begin[t + 1] - b;
         BinNode& r = bn[t];
@@ -142,6 +147,8 @@ __global__ void k_roots(const float* boxes, const int* tree_begin, int num_trees
         } else if (n <= kSmall) {
             for (int i = 0; i < n; ++i) ord_fin[b + i] = b + i;
             small[atomicAdd(n_small, 1)] = t;
+        } else if (n <= kMedium) {
+            medium[atomicAdd(n_medium, 1)] = unsigned(t);  // its order is in buffer 0
         } else {
             large[atomicAdd(n_large, 1)] = t;
         }
@@ -330,6 +337,78 @@ __global__ void __launch_bounds__(kBlock) k_bin(const float* boxes, const int* o
 // prefix union over lanes 0..b, those right of it a suffix union over lanes b+1..31 (empty
 // bins contribute nothing), so every candidate's cost is the host's value exactly.
 constexpr int kSplitWarps = 4;
+
+// The sweep of one axis: lane b holds bin b's count n and box; (best, bsp, bnl) take the lane's
+// split if it is the axis's candidate of lower cost than best. Whole warps call it.
+__device__ __forceinline__ void sweep_axis(int a, int n, const float* lo, const float* hi, double& best, int& bax,
+                                           int& bsp, int& bnl) {
+    const int lane = threadIdx.x & 31;
+    // inclusive prefix (left side) and inclusive suffix unions over the lanes
+    float pl[3], ph[3], ql[3], qh[3];
+    int pc = n, qc = n;
+    for (int d = 0; d < 3; ++d) {
+        pl[d] = ql[d] = lo[d];
+        ph[d] = qh[d] = hi[d];
+    }
+    for (int off = 1; off < 32; off <<= 1) {
+        const int uc = __shfl_up_sync(FULL, pc, off), dc = __shfl_down_sync(FULL, qc, off);
+        float ul[3], uh[3], dl[3], dh[3];
+        for (int d = 0; d < 3; ++d) {
+            ul[d] = __shfl_up_sync(FULL, pl[d], off);
+            uh[d] = __shfl_up_sync(FULL, ph[d], off);
+            dl[d] = __shfl_down_sync(FULL, ql[d], off);
+            dh[d] = __shfl_down_sync(FULL, qh[d], off);
+        }
+        if (lane >= off) {
+            pc += uc;
+            for (int d = 0; d < 3; ++d) {
+                pl[d] = fminf(pl[d], ul[d]);
+                ph[d] = fmaxf(ph[d], uh[d]);
+            }
+        }
+        if (lane + off < 32) {
+            qc += dc;
+            for (int d = 0; d < 3; ++d) {
+                ql[d] = fminf(ql[d], dl[d]);
+                qh[d] = fmaxf(qh[d], dh[d]);
+            }
+        }
+    }
+    // right side of a split after bin b: the suffix from b + 1
+    int rc = __shfl_down_sync(FULL, qc, 1);
+    float rl[3], rh[3];
+    for (int d = 0; d < 3; ++d) {
+        rl[d] = __shfl_down_sync(FULL, ql[d], 1);
+        rh[d] = __shfl_down_sync(FULL, qh[d], 1);
+    }
+    if (lane == 31) rc = 0;
+    if (n > 0 && rc > 0) {
+        const double c = sah(area(pl, ph), pc, area(rl, rh), rc);
+        if (c < best) {  // axes ascend, so an earlier axis keeps a tie
+            best = c;
+            bax = a;
+            bsp = lane;
+            bnl = pc;
+        }
+    }
+}
+
+// Of all lanes' candidates the lowest (cost, axis, bin), in every lane.
+__device__ __forceinline__ void best_split(double& best, int& bax, int& bsp, int& bnl) {
+    for (int off = 16; off > 0; off >>= 1) {
+        const double ob = __shfl_xor_sync(FULL, best, off);
+        const int oa = __shfl_xor_sync(FULL, bax, off);
+        const int os = __shfl_xor_sync(FULL, bsp, off);
+        const int on = __shfl_xor_sync(FULL, bnl, off);
+        if (ob < best || (ob == best && (oa < bax || (oa == bax && os < bsp)))) {
+            best = ob;
+            bax = oa;
+            bsp = os;
+            bnl = on;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(32 * kSplitWarps) k_split(const int* level, const int* n_level_ptr, const BinNode* bn,
                                                              Slot* slots, const unsigned* bin_cnt,
                                                              const unsigned* bin_lo, const unsigned* bin_hi) {
@@ -349,67 +428,9 @@ __global__ void __launch_bounds__(32 * kSplitWarps) k_split(const int* level, co
                 lo[d] = n ? fval(bin_lo[g * 3 + d]) : FLT_MAX;
                 hi[d] = n ? fval(bin_hi[g * 3 + d]) : -FLT_MAX;
             }
-            // inclusive prefix (left side) and inclusive suffix unions over the lanes
-            float pl[3], ph[3], ql[3], qh[3];
-            int pc = n, qc = n;
-            for (int d = 0; d < 3; ++d) {
-                pl[d] = ql[d] = lo[d];
-                ph[d] = qh[d] = hi[d];
-            }
-            for (int off = 1; off < 32; off <<= 1) {
-                const int uc = __shfl_up_sync(FULL, pc, off), dc = __shfl_down_sync(FULL, qc, off);
-                float ul[3], uh[3], dl[3], dh[3];
-                for (int d = 0; d < 3; ++d) {
-                    ul[d] = __shfl_up_sync(FULL, pl[d], off);
-                    uh[d] = __shfl_up_sync(FULL, ph[d], off);
-                    dl[d] = __shfl_down_sync(FULL, ql[d], off);
-                    dh[d] = __shfl_down_sync(FULL, qh[d], off);
-                }
-                if (lane >= off) {
-                    pc += uc;
-                    for (int d = 0; d < 3; ++d) {
-                        pl[d] = fminf(pl[d], ul[d]);
-                        ph[d] = fmaxf(ph[d], uh[d]);
-                    }
-                }
-                if (lane + off < 32) {
-                    qc += dc;
-                    for (int d = 0; d < 3; ++d) {
-                        ql[d] = fminf(ql[d], dl[d]);
-                        qh[d] = fmaxf(qh[d], dh[d]);
-                    }
-                }
-            }
-            // right side of a split after bin b: the suffix from b + 1
-            int rc = __shfl_down_sync(FULL, qc, 1);
-            float rl[3], rh[3];
-            for (int d = 0; d < 3; ++d) {
-                rl[d] = __shfl_down_sync(FULL, ql[d], 1);
-                rh[d] = __shfl_down_sync(FULL, qh[d], 1);
-            }
-            if (lane == 31) rc = 0;
-            if (n > 0 && rc > 0) {
-                const double c = sah(area(pl, ph), pc, area(rl, rh), rc);
-                if (c < best) {  // axes ascend, so an earlier axis keeps a tie
-                    best = c;
-                    bax = a;
-                    bsp = lane;
-                    bnl = pc;
-                }
-            }
+            sweep_axis(a, n, lo, hi, best, bax, bsp, bnl);
         }
-        for (int off = 16; off > 0; off >>= 1) {
-            const double ob = __shfl_xor_sync(FULL, best, off);
-            const int oa = __shfl_xor_sync(FULL, bax, off);
-            const int os = __shfl_xor_sync(FULL, bsp, off);
-            const int on = __shfl_xor_sync(FULL, bnl, off);
-            if (ob < best || (ob == best && (oa < bax || (oa == bax && os < bsp)))) {
-                best = ob;
-                bax = oa;
-                bsp = os;
-                bnl = on;
-            }
-        }
+        best_split(best, bax, bsp, bnl);
         if (lane == 0) {
             int axis = bax < 3 ? bax : -1;
             if (axis >= 0 && (bnl <= 0 || bnl >= nd.count)) axis = -1;
@@ -533,13 +554,14 @@ __global__ void __launch_bounds__(kBlock) k_scatter(const float* boxes, const in
 }
 
 // Children of the level's nodes: ids next_id + 2 s and + 1; leaves take their primitive's box
-// at once, small children go to the warp list (their range copied to the final order), large
-// children to the next level.
+// at once, small children go to the warp list (their range copied to the final order), medium ones
+// to the block list (with the order buffer their range stays in), large children to the next level.
 // Child ids continue from *next_id (k_level_advance moves it on); ids past bn_cap set *err
 // and the level stops there.
 __global__ void k_children(const float* boxes, const int* ord_next, int* ord_fin, const int* level,
                            const int* n_level_ptr, BinNode* bn, const Slot* slots, const int* next_id_ptr,
-                           int bn_cap, int* err, int* large_next, int* n_large_next, int* small, int* n_small) {
+                           int bn_cap, int* err, int* large_next, int* n_large_next, unsigned* medium, int* n_medium,
+                           unsigned buffer, int* small, int* n_small) {
     const int n_level = *n_level_ptr, next_id = *next_id_ptr;
     if (n_level > 0 && next_id + 2 * n_level > bn_cap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *err = 1;
@@ -565,10 +587,231 @@ __global__ void k_children(const float* boxes, const int* ord_next, int* ord_fin
             } else if (cnt[k] <= kSmall) {
                 for (int i = 0; i < cnt[k]; ++i) ord_fin[beg[k] + i] = ord_next[beg[k] + i];
                 small[atomicAdd(n_small, 1)] = ids[k];
+            } else if (cnt[k] <= kMedium) {
+                medium[atomicAdd(n_medium, 1)] = unsigned(ids[k]) | buffer << 31;
             } else {
                 large_next[atomicAdd(n_large_next, 1)] = ids[k];
             }
         }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// binary stage: subtrees of at most kMedium primitives down to kSmall, one block each
+// ---------------------------------------------------------------------------------------------
+
+// The passes of one level of large nodes (bounds, bins, sweep, stable partition) on a node in
+// shared memory, node after node: below kMedium primitives the levels' eleven launches each, with
+// a few us of work, were the larger part of the binary stage (1M triangles: 9 of its 25 levels and
+// 4.0 ms of kernels; now 16 levels, 2.1 ms, and 0.59 ms here).
+// 31 KB of shared memory, so seven blocks share an SM and hide one another's barriers.
+__global__ void __launch_bounds__(kBlock) k_medium(const float* boxes, const int* ord0, const int* ord1,
+                                                   const unsigned* medium, const int* n_medium_ptr, BinNode* bn,
+                                                   int bn_cap, int* next_id, int* err, int* ord_fin, int* small,
+                                                   int* n_small) {
+    constexpr int kPer = kMedium / kBlock;
+    constexpr int kWarps = kBlock / 32;
+    __shared__ float sb[6][kMedium];
+    __shared__ int sid[kMedium];
+    __shared__ unsigned cnt[3 * kBins], blo[3 * kBins * 3], bhi[3 * kBins * 3];
+    __shared__ unsigned red[12];
+    __shared__ double s_cost[3], k1[3];
+    __shared__ float clo[3];
+    __shared__ int s_bin[3], s_nl[3], live[3], wsum[kWarps], s_ids;
+    // nodes to split: the smaller child is taken first, so few wait
+    __shared__ int st_node[16], st_at[16], st_n[16];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n_medium = *n_medium_ptr;
+    for (int w = blockIdx.x; w < n_medium; w += gridDim.x) {
+        const int root = int(medium[w] & 0x7fffffffu);
+        const int* ord = (medium[w] >> 31) ? ord1 : ord0;
+        const int base = bn[root].begin, n0 = min(bn[root].count, kMedium);
+        for (int i = tid; i < n0; i += kBlock) {
+            const int p = ord[base + i];
+            float lo[3], hi[3];
+            load_prim(boxes, p, lo, hi);
+            sid[i] = p;
+            for (int a = 0; a < 3; ++a) {
+                sb[a][i] = lo[a];
+                sb[3 + a][i] = hi[a];
+            }
+        }
+        int sp = 1;
+        if (tid == 0) {
+            st_node[0] = root;
+            st_at[0] = 0;
+            st_n[0] = n0;
+        }
+        __syncthreads();
+        while (sp > 0) {
+            --sp;
+            const int node = st_node[sp], at = st_at[sp], n = st_n[sp];
+            // bounds
+            if (tid < 12) red[tid] = (tid < 3 || (tid >= 6 && tid < 9)) ? 0xffffffffu : 0u;
+            for (int b = tid; b < 3 * kBins; b += kBlock) {
+                cnt[b] = 0;
+                for (int d = 0; d < 3; ++d) {
+                    blo[b * 3 + d] = 0xffffffffu;
+                    bhi[b * 3 + d] = 0u;
+                }
+            }
+            unsigned r[12];
+            for (int k = 0; k < 12; ++k) r[k] = (k < 3 || (k >= 6 && k < 9)) ? 0xffffffffu : 0u;
+            for (int i = tid; i < n; i += kBlock)
+                for (int a = 0; a < 3; ++a) {
+                    const float l = sb[a][at + i], h = sb[3 + a][at + i], c = cen(l, h);
+                    r[a] = min(r[a], fkey(l));
+                    r[3 + a] = max(r[3 + a], fkey(h));
+                    r[6 + a] = min(r[6 + a], fkey(c));
+                    r[9 + a] = max(r[9 + a], fkey(c));
+                }
+            __syncthreads();
+            if (warp * 32 < n) {
+                for (int k = 0; k < 12; ++k) {
+                    const bool mn = k < 3 || (k >= 6 && k < 9);
+                    r[k] = mn ? __reduce_min_sync(FULL, r[k]) : __reduce_max_sync(FULL, r[k]);
+                    if (lane == 0) {
+                        if (mn) atomicMin(&red[k], r[k]);
+                        else atomicMax(&red[k], r[k]);
+                    }
+                }
+            }
+            __syncthreads();
+            if (tid < 3) {
+                bn[node].lo[tid] = fval(red[tid]);
+                bn[node].hi[tid] = fval(red[3 + tid]);
+                const float cl = fval(red[6 + tid]), ch = fval(red[9 + tid]);
+                const double ext = __dsub_rn(double(ch), double(cl));
+                clo[tid] = cl;
+                live[tid] = ext > 0.0;
+                k1[tid] = ext > 0.0 ? __ddiv_rn(double(kBins), ext) : 0.0;
+            }
+            __syncthreads();
+            // bins
+            for (int i = tid; i < n; i += kBlock) {
+                unsigned lk[3], hk[3];
+                for (int d = 0; d < 3; ++d) {
+                    lk[d] = fkey(sb[d][at + i]);
+                    hk[d] = fkey(sb[3 + d][at + i]);
+                }
+                for (int a = 0; a < 3; ++a) {
+                    if (!live[a]) continue;
+                    const int b = a * kBins + bin_of(cen(sb[a][at + i], sb[3 + a][at + i]), clo[a], k1[a]);
+                    atomicAdd(&cnt[b], 1u);
+                    for (int d = 0; d < 3; ++d) {
+                        atomicMin(&blo[b * 3 + d], lk[d]);
+                        atomicMax(&bhi[b * 3 + d], hk[d]);
+                    }
+                }
+            }
+            __syncthreads();
+            // sweep: one warp per axis, lane = bin
+            if (warp < 3) {
+                double best = DBL_MAX;
+                int bax = 3, bsp = kBins, bnl = 0;
+                if (live[warp]) {
+                    const int g = warp * kBins + lane;
+                    const int c = int(cnt[g]);
+                    float lo[3], hi[3];
+                    for (int d = 0; d < 3; ++d) {
+                        lo[d] = c ? fval(blo[g * 3 + d]) : FLT_MAX;
+                        hi[d] = c ? fval(bhi[g * 3 + d]) : -FLT_MAX;
+                    }
+                    sweep_axis(warp, c, lo, hi, best, bax, bsp, bnl);
+                    best_split(best, bax, bsp, bnl);
+                }
+                if (lane == 0) {
+                    s_cost[warp] = bax < 3 ? best : DBL_MAX;
+                    s_bin[warp] = bax < 3 ? bsp : -1;
+                    s_nl[warp] = bnl;
+                }
+            }
+            if (tid == 96) s_ids = atomicAdd(next_id, 2);
+            __syncthreads();
+            int axis = -1;
+            for (int a = 0; a < 3; ++a)
+                if (s_bin[a] >= 0 && (axis < 0 || s_cost[a] < s_cost[axis])) axis = a;
+            if (axis >= 0 && (s_nl[axis] <= 0 || s_nl[axis] >= n)) axis = -1;
+            const int split = axis >= 0 ? s_bin[axis] : -1;
+            const int nl = axis >= 0 ? s_nl[axis] : n / 2;
+            const int id = s_ids;
+            if (id + 2 > bn_cap) {
+                if (tid == 0) *err = 1;
+                break;
+            }
+            // stable partition: thread t owns positions t * per .. t * per + per - 1, in registers
+            const int per = (n + kBlock - 1) / kBlock;
+            float pb[kPer][6];
+            int pp[kPer];
+            unsigned lmask = 0;
+            int mine = 0;
+            for (int k = 0; k < kPer; ++k) {
+                const int i = tid * per + k;
+                if (k >= per || i >= n) break;
+                pp[k] = sid[at + i];
+                for (int d = 0; d < 6; ++d) pb[k][d] = sb[d][at + i];
+                const bool left = axis < 0 ? i < nl : bin_of(cen(sb[axis][at + i], sb[3 + axis][at + i]), clo[axis], k1[axis]) <= split;
+                if (left) {
+                    lmask |= 1u << k;
+                    ++mine;
+                }
+            }
+            int incl = mine;
+            for (int off = 1; off < 32; off <<= 1) {
+                const int v = __shfl_up_sync(FULL, incl, off);
+                if (lane >= off) incl += v;
+            }
+            if (lane == 31) wsum[warp] = incl;
+            __syncthreads();
+            int lrank = incl - mine;
+            for (int v = 0; v < warp; ++v) lrank += wsum[v];
+            for (int k = 0; k < kPer; ++k) {
+                const int i = tid * per + k;
+                if (k >= per || i >= n) break;
+                const bool left = (lmask >> k) & 1u;
+                const int to = at + (left ? lrank : nl + (i - lrank));
+                lrank += left ? 1 : 0;
+                sid[to] = pp[k];
+                for (int d = 0; d < 6; ++d) sb[d][to] = pb[k][d];
+            }
+            __syncthreads();
+            // children: leaves and small subtrees leave the block, the others wait here
+            if (tid == 0) {
+                bn[node].left = id;
+                bn[node].right = id + 1;
+            }
+            const int first = nl > n - nl ? 0 : 1;  // the larger child waits below the smaller
+            for (int j = 0; j < 2; ++j) {
+                const int k = j == 0 ? first : 1 - first;
+                const int cat = k ? at + nl : at, cn = k ? n - nl : nl;
+                if (tid == 0) {
+                    BinNode& ch = bn[id + k];
+                    ch.begin = base + cat;
+                    ch.count = cn;
+                    ch.left = ch.right = -1;
+                    if (cn == 1)
+                        for (int a = 0; a < 3; ++a) {
+                            ch.lo[a] = sb[a][cat];
+                            ch.hi[a] = sb[3 + a][cat];
+                        }
+                    else if (cn <= kSmall) small[atomicAdd(n_small, 1)] = id + k;
+                }
+                if (cn <= kSmall) {
+                    if (tid < cn) ord_fin[base + cat + tid] = sid[cat + tid];
+                } else if (sp < 16) {
+                    if (tid == 0) {
+                        st_node[sp] = id + k;
+                        st_at[sp] = cat;
+                        st_n[sp] = cn;
+                    }
+                    ++sp;
+                } else if (tid == 0) {
+                    *err = 1;  // cannot be: each waiting node is at least as large as all above it
+                }
+            }
+            __syncthreads();
+        }
+        __syncthreads();
     }
 }
 
@@ -587,6 +830,9 @@ __device__ __forceinline__ float wmax(float v) {
     return v;
 }
 
+// All nodes of one depth of the subtree are split together: lanes lb .. lb + n - 1 hold a node's
+// primitives in order, so every step is a segmented warp operation, and a subtree takes its depth
+// in steps instead of its node count (1M triangles: 1.15 ms node by node, 0.48 so).
 __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const float* boxes, const int* small, const int* n_small_ptr,
                                                             BinNode* bn, int* ord_fin, int* bn_next) {
     __shared__ int perm[kSmallWarps][32];
@@ -594,89 +840,99 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const float* boxes, 
     const int n_small = *n_small_ptr;
     const unsigned lt = (1u << lane) - 1u;
     for (int w = blockIdx.x * kSmallWarps + wib; w < n_small; w += gridDim.x * kSmallWarps) {
-        const int root = small[w];
-        const int begin0 = bn[root].begin, cnt0 = min(bn[root].count, kSmall);   // 2 .. kSmall
+        int node = small[w];  // the node of this lane's segment
+        const int begin0 = bn[node].begin, cnt0 = min(bn[node].count, kSmall);   // 2 .. kSmall
         int pid = -1;
         float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, c[3] = {0.f, 0.f, 0.f};
+        int lb = 0, n = cnt0;  // the lane's segment; lanes past the subtree are segments of their own
         if (lane < cnt0) {
             pid = ord_fin[begin0 + lane];
             load_prim(boxes, pid, lo, hi);
             for (int a = 0; a < 3; ++a) c[a] = cen(lo[a], hi[a]);
+        } else {
+            lb = lane;
+            n = 1;
         }
         int next = 0;
         if (lane == 0) next = atomicAdd(bn_next, 2 * cnt0 - 2);
         next = __shfl_sync(FULL, next, 0);
-        // stack entry k lives in lane k's registers
-        int st_node = 0, st_lb = 0, st_n = 0;
-        int sp = 0;
-        if (lane == 0) {
-            st_node = root;
-            st_lb = 0;
-            st_n = cnt0;
-        }
-        sp = 1;
-        while (sp > 0) {
-            --sp;
-            const int node = __shfl_sync(FULL, st_node, sp);
-            const int lb = __shfl_sync(FULL, st_lb, sp);
-            const int n = __shfl_sync(FULL, st_n, sp);
-            const bool in = lane >= lb && lane < lb + n;
-            const unsigned inmask = __ballot_sync(FULL, in);
-            // box and centroid bounds over the node's lanes
+        while (true) {
+            const bool in = n > 1;
+            if (!__any_sync(FULL, in)) break;
+            const bool leader = in && lane == lb;
+            const int end = lb + n - 1;  // last lane of the segment
+            // box and centroid bounds: segmented inclusive scans, then the last lane's value
             float nlo[3], nhi[3], clo[3], chi[3];
             for (int a = 0; a < 3; ++a) {
-                nlo[a] = wmin(in ? lo[a] : FLT_MAX);
-                nhi[a] = wmax(in ? hi[a] : -FLT_MAX);
-                clo[a] = wmin(in ? c[a] : FLT_MAX);
-                chi[a] = wmax(in ? c[a] : -FLT_MAX);
-            }
-            if (lane == 0) {
-                BinNode& nd = bn[node];
-                for (int a = 0; a < 3; ++a) {
-                    nd.lo[a] = nlo[a];
-                    nd.hi[a] = nhi[a];
+                nlo[a] = lo[a];
+                nhi[a] = hi[a];
+                clo[a] = chi[a] = c[a];
+                for (int off = 1; off < 32; off <<= 1) {
+                    const float x0 = __shfl_up_sync(FULL, nlo[a], off), x1 = __shfl_up_sync(FULL, nhi[a], off);
+                    const float x2 = __shfl_up_sync(FULL, clo[a], off), x3 = __shfl_up_sync(FULL, chi[a], off);
+                    if (lane - off >= lb) {
+                        nlo[a] = fminf(nlo[a], x0);
+                        nhi[a] = fmaxf(nhi[a], x1);
+                        clo[a] = fminf(clo[a], x2);
+                        chi[a] = fmaxf(chi[a], x3);
+                    }
                 }
+                nlo[a] = __shfl_sync(FULL, nlo[a], end);
+                nhi[a] = __shfl_sync(FULL, nhi[a], end);
+                clo[a] = __shfl_sync(FULL, clo[a], end);
+                chi[a] = __shfl_sync(FULL, chi[a], end);
             }
-            int newpos = lane;  // position after the partition, for lanes of the node
-            int mid;
-            if (n == 2) {
-                // the first axis with a centroid extent decides: the smaller centroid goes left
-                bool swap = false;
+            if (leader)
                 for (int a = 0; a < 3; ++a) {
-                    if (!(__dsub_rn(double(chi[a]), double(clo[a])) > 0.0)) continue;
-                    const float c0 = __shfl_sync(FULL, c[a], lb), c1 = __shfl_sync(FULL, c[a], lb + 1);
+                    bn[node].lo[a] = nlo[a];
+                    bn[node].hi[a] = nhi[a];
+                }
+            int newpos = lane;      // position after the partition
+            int mid = lb + n / 2;   // coincident centroids: halve by position
+            // two primitives: the first axis with a centroid extent decides, the smaller centroid
+            // goes left
+            bool swap = false, decided = false;
+            for (int a = 0; a < 3; ++a) {
+                const float c0 = __shfl_sync(FULL, c[a], lb), c1 = __shfl_sync(FULL, c[a], end);
+                if (!decided && __dsub_rn(double(chi[a]), double(clo[a])) > 0.0) {
                     swap = c1 < c0;
-                    break;
+                    decided = true;
                 }
-                if (swap && in) newpos = lane == lb ? lb + 1 : lb;
+            }
+            if (n == 2) {
+                if (swap) newpos = lane == lb ? lb + 1 : lb;
                 mid = lb + 1;
-            } else {
-                double k1[3];
+            }
+            const bool sahn = n > 2;
+            if (__any_sync(FULL, sahn)) {
+                const int longest = __reduce_max_sync(FULL, sahn ? n : 0);
+                int bin[3] = {0, 0, 0};
                 int live = 0;
                 for (int a = 0; a < 3; ++a) {
                     const double ext = __dsub_rn(double(chi[a]), double(clo[a]));
-                    k1[a] = ext > 0.0 ? __ddiv_rn(double(kBins), ext) : 0.0;
-                    if (ext > 0.0) live |= 1 << a;
+                    if (sahn && ext > 0.0) {
+                        live |= 1 << a;
+                        bin[a] = bin_of(c[a], clo[a], __ddiv_rn(double(kBins), ext));
+                    }
                 }
-                int bin[3] = {0, 0, 0};
-                for (int a = 0; a < 3; ++a)
-                    if (in && ((live >> a) & 1)) bin[a] = bin_of(c[a], clo[a], k1[a]);
                 // each lane evaluates the split after its own bin on every live axis
                 double best = DBL_MAX;
                 int bax = 3, bsp = kBins, bnl = 0;
                 bool any = false;
                 for (int a = 0; a < 3; ++a) {
-                    if (!((live >> a) & 1)) continue;
+                    if (!__any_sync(FULL, (live >> a) & 1)) continue;
                     float l_lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, l_hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
                     float r_lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, r_hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
                     int nl = 0, nr = 0;
-                    for (int m = lb; m < lb + n; ++m) {
+                    for (int t = 0; t < longest; ++t) {
+                        const int m = min(lb + t, end);
                         const int bm = __shfl_sync(FULL, bin[a], m);
                         float mlo[3], mhi[3];
                         for (int d = 0; d < 3; ++d) {
                             mlo[d] = __shfl_sync(FULL, lo[d], m);
                             mhi[d] = __shfl_sync(FULL, hi[d], m);
                         }
+                        if (t >= n) continue;
                         if (bm <= bin[a]) {
                             for (int d = 0; d < 3; ++d) {
                                 l_lo[d] = fminf(l_lo[d], mlo[d]);
@@ -691,7 +947,7 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const float* boxes, 
                             ++nr;
                         }
                     }
-                    if (in && nr > 0) {
+                    if (((live >> a) & 1) && nr > 0) {
                         const double cst = sah(area(l_lo, l_hi), nl, area(r_lo, r_hi), nr);
                         if (!any || cst < best) {  // axes ascend, so the first wins ties
                             best = cst;
@@ -702,34 +958,36 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const float* boxes, 
                         }
                     }
                 }
-                // warp arg-min over (cost, axis, bin)
-                for (int off = 16; off > 0; off >>= 1) {
-                    const double ob = __shfl_xor_sync(FULL, best, off);
-                    const int oa = __shfl_xor_sync(FULL, bax, off);
-                    const int os = __shfl_xor_sync(FULL, bsp, off);
-                    const int on = __shfl_xor_sync(FULL, bnl, off);
-                    const bool take = ob < best || (ob == best && (oa < bax || (oa == bax && os < bsp)));
-                    if (take) {
+                // the segment's lowest (cost, axis, bin)
+                for (int off = 1; off < 32; off <<= 1) {
+                    const double ob = __shfl_up_sync(FULL, best, off);
+                    const int oa = __shfl_up_sync(FULL, bax, off);
+                    const int os = __shfl_up_sync(FULL, bsp, off);
+                    const int on = __shfl_up_sync(FULL, bnl, off);
+                    if (lane - off >= lb && (ob < best || (ob == best && (oa < bax || (oa == bax && os < bsp))))) {
                         best = ob;
                         bax = oa;
                         bsp = os;
                         bnl = on;
                     }
                 }
-                if (bax < 3 && bnl > 0 && bnl < n) {
-                    const bool l = in && bin[bax] <= bsp;
-                    const unsigned lm = __ballot_sync(FULL, l);
-                    const int nl = __popc(lm);
-                    if (in) newpos = l ? lb + __popc(lm & lt) : lb + nl + __popc(inmask & ~lm & lt);
+                bax = __shfl_sync(FULL, bax, end);
+                bsp = __shfl_sync(FULL, bsp, end);
+                bnl = __shfl_sync(FULL, bnl, end);
+                const bool part = sahn && bax < 3 && bnl > 0 && bnl < n;
+                const int mybin = bax == 0 ? bin[0] : (bax == 1 ? bin[1] : bin[2]);
+                const unsigned lm = __ballot_sync(FULL, part && mybin <= bsp);
+                if (part) {
+                    const unsigned seg = (n == 32 ? FULL : (1u << n) - 1u) << lb;
+                    const int nl = __popc(lm & seg);
+                    newpos = (lm >> lane) & 1u ? lb + __popc(lm & seg & lt) : lb + nl + __popc(~lm & seg & lt);
                     mid = lb + nl;
-                } else {
-                    mid = lb + n / 2;  // coincident centroids: halve by position
                 }
             }
-            // apply the permutation (lanes of the node move to newpos)
-            if (in) perm[wib][newpos] = lane;
+            // apply the permutation (lanes move to newpos)
+            perm[wib][newpos] = lane;
             __syncwarp();
-            const int src = in ? perm[wib][lane] : lane;
+            const int src = perm[wib][lane];
             __syncwarp();
             pid = __shfl_sync(FULL, pid, src);
             for (int a = 0; a < 3; ++a) {
@@ -737,38 +995,32 @@ __global__ void __launch_bounds__(32 * kSmallWarps) k_small(const float* boxes, 
                 hi[a] = __shfl_sync(FULL, hi[a], src);
                 c[a] = __shfl_sync(FULL, c[a], src);
             }
-            // children
-            const int ids[2] = {next, next + 1};
-            next += 2;
-            const int clb[2] = {lb, mid};
-            const int cn[2] = {mid - lb, lb + n - mid};
-            if (lane == 0) {
-                bn[node].left = ids[0];
-                bn[node].right = ids[1];
-            }
-            for (int k = 0; k < 2; ++k) {
-                if (lane == 0) {
-                    BinNode& ch = bn[ids[k]];
-                    ch.begin = begin0 + clb[k];
-                    ch.count = cn[k];
-                    ch.left = ch.right = -1;
+            // children: two ids per segment
+            const unsigned leaders = __ballot_sync(FULL, leader);
+            const int id = next + 2 * __popc(leaders & ((1u << lb) - 1u));
+            next += 2 * __popc(leaders);
+            if (in) {
+                const bool right = lane >= mid;
+                if (leader) {
+                    bn[node].left = id;
+                    bn[node].right = id + 1;
                 }
-                if (cn[k] == 1) {
-                    if (lane == clb[k]) {
-                        BinNode& ch = bn[ids[k]];
+                const int e = lb + n;
+                lb = right ? mid : lb;
+                n = right ? e - mid : mid - lb;
+                node = id + (right ? 1 : 0);
+                if (lane == lb) {
+                    BinNode& ch = bn[node];
+                    ch.begin = begin0 + lb;
+                    ch.count = n;
+                    ch.left = ch.right = -1;
+                    if (n == 1) {
                         for (int a = 0; a < 3; ++a) {
                             ch.lo[a] = lo[a];
                             ch.hi[a] = hi[a];
                         }
                         ord_fin[begin0 + lane] = pid;
                     }
-                } else {
-                    if (lane == sp) {
-                        st_node = ids[k];
-                        st_lb = clb[k];
-                        st_n = cn[k];
-                    }
-                    ++sp;
                 }
             }
         }
@@ -784,254 +1036,279 @@ struct Item {
     int tree;
 };
 
-// The items a launch works on: [off, off + count) of the level arrays. With lvl set, both come
-// from the device level table (lvl[2 l], lvl[2 l + 1]), so that levels are launched back to back
-// without the host reading their sizes; otherwise off = 0 and count = n.
-struct Span {
-    const int* lvl;
-    int l;
-    int n;
-    __device__ int off() const { return lvl ? lvl[2 * l] : 0; }
-    __device__ int count() const { return lvl ? lvl[2 * l + 1] : n; }
-};
+// Look-back words of the collapse: bits 62-63 the state (0 not yet, 1 the tile's own counts, 2 those
+// of it and all earlier tiles of the level), then the leaf and internal children, 31 bits each.
+using TileWord = unsigned long long;
+constexpr TileWord kOwn = TileWord(1) << 62, kPrefix = TileWord(2) << 62, kCounts = kOwn - 1;
+constexpr TileWord kIntMask = (TileWord(1) << 31) - 1;
+// Polls of a word before a look-back gives up (err): tiles are taken in order by running blocks.
+constexpr int kPollLimit = 1 << 22;
+constexpr int kMaxLevels = 120;  // 8-wide levels
+constexpr int kColThreads = 256;
+constexpr int kColItems = kColThreads / 8;  // items of a tile, eight lanes each
 
-// One 8-wide node per item: its children, slots, quantised boxes (child_base and tri_base are
-// placed later), the binary ids of its internal children and the primitives of its leaf slots,
-// both in slot order.
-__global__ void k_collapse(Span sp, const Item* items_all, const BinNode* bn, const int* ord_fin, BVH8Node* tmp_all,
-                           int* n_int_all, int* n_leaf_all, int* child_bn_all, int* leaf_prim_all) {
-    const int o = sp.off(), n_items = sp.count();
+// One level of 8-wide nodes: level l of the table (lvl[2 l]: offset of its items, lvl[2 l + 1]: their
+// number). Per item: its children, slots and quantised boxes (child_base and tri_base are placed
+// later) and the primitives of its leaf slots in slot order; cs and ls: internal children and leaf
+// slots of the level's earlier items; the next level's items, in order, right after this level's,
+// and its entry in the table. Past the capacity it is left empty and err is set.
+// Eight lanes hold an item's children, one each: a thread per item kept them in local memory and
+// took about 100 us a level however few items it had, and the places took eight more launches
+// (1M triangles, 11 levels: 1.08 ms and 88 launches of 0.4 ms; 0.46 ms so).
+__global__ void __launch_bounds__(kColThreads) k_collapse(int* lvl, int l, Item* items_all, const BinNode* bn,
+                                                          const int* ord_fin, BVH8Node* tmp_all, int* n_leaf_all,
+                                                          int* cs_all, int* ls_all, int* leaf_prim_all,
+                                                          TileWord* words_all, int* tile_ctr, long long cap, int* err) {
+    __shared__ BVH8Node s_node[kColItems];
+    __shared__ TileWord s_count[kColItems];
+    __shared__ int s_tile;
+    const int o = lvl[2 * l], n_items = lvl[2 * l + 1];
+    const int tiles = (n_items + kColItems - 1) / kColItems;
     const Item* items = items_all + o;
-    BVH8Node* tmp = tmp_all + o;
-    int *n_int = n_int_all + o, *n_leaf = n_leaf_all + o;
-    int *child_bn = child_bn_all + size_t(o) * 8, *leaf_prim = leaf_prim_all + size_t(o) * 8;
-    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n_items; it += gridDim.x * blockDim.x) {
-        const BinNode& b = bn[items[it].bnode];
-        int ch[8];
-        int nch = 0;
+    TileWord* words = words_all + o / kColItems + l;
+    const int lane = threadIdx.x & 31, j = threadIdx.x & 7, g = threadIdx.x >> 3, g0 = lane & ~7;
+    while (true) {
+        if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr + l, 1);
+        __syncthreads();
+        const int tile = s_tile;
+        if (tile >= tiles) break;
+        const int it = tile * kColItems + g;
+        const bool on = it < n_items;
+        const Item item = on ? items[it] : Item{0, 0};
+        const BinNode b = bn[item.bnode];
+        // children: lane j holds child j
+        int nch = 1, id = -1;
+        bool open = false;
         if (b.left < 0 || b.count <= kMaxLeafPrims) {
-            ch[nch++] = items[it].bnode;
+            if (j == 0) id = item.bnode;
         } else {
-            ch[nch++] = b.left;
-            ch[nch++] = b.right;
-            while (nch < 8) {
-                int pick = -1;
-                double pa = -1.0;
-                for (int k = 0; k < nch; ++k) {
-                    const BinNode& c = bn[ch[k]];
-                    if (c.left < 0 || c.count <= kMaxLeafPrims) continue;
-                    const double a = area(c.lo, c.hi);
-                    if (a > pa) {
-                        pa = a;
-                        pick = k;
-                    }
+            nch = 2;
+            if (j < 2) id = j == 0 ? b.left : b.right;
+            open = true;
+        }
+        BinNode c = bn[id < 0 ? 0 : id];
+        for (int round = 0; round < 6; ++round) {  // two children at first, eight at most
+            // the child of largest area that is no leaf, the first of equals
+            double pa = -1.0;
+            int pick = -1;
+            if (open && j < nch && c.left >= 0 && c.count > kMaxLeafPrims) {
+                const double a = area(c.lo, c.hi);
+                if (a > pa) {
+                    pa = a;
+                    pick = j;
                 }
-                if (pick < 0) break;
-                const int c = ch[pick];
-                ch[pick] = bn[c].left;
-                ch[nch++] = bn[c].right;
             }
+            for (int off = 1; off < 8; off <<= 1) {
+                const double oa = __shfl_xor_sync(FULL, pa, off);
+                const int op = __shfl_xor_sync(FULL, pick, off);
+                if (oa > pa || (oa == pa && op >= 0 && (pick < 0 || op < pick))) {
+                    pa = oa;
+                    pick = op;
+                }
+            }
+            pick = __shfl_sync(FULL, pick, g0);
+            open = open && pick >= 0;
+            const int from = g0 + (pick < 0 ? 0 : pick);
+            const int cl = __shfl_sync(FULL, c.left, from), cr = __shfl_sync(FULL, c.right, from);
+            if (open) {
+                if (j == pick || j == nch) {
+                    id = j == pick ? cl : cr;
+                    c = bn[id];
+                }
+                ++nch;
+            }
+            if (!__any_sync(FULL, open)) break;
         }
         // slots by centroid octant around the node centre, cheapest (child, slot) pairs first
-        float ctr[3];
-        for (int a = 0; a < 3; ++a) ctr[a] = cen(b.lo[a], b.hi[a]);
-        double cost[8][8];
-        for (int k = 0; k < nch; ++k) {
-            const BinNode& c = bn[ch[k]];
-            double d[3];
-            for (int a = 0; a < 3; ++a)
-                d[a] = __dsub_rn(__dmul_rn(0.5, __dadd_rn(double(c.lo[a]), double(c.hi[a]))), double(ctr[a]));
-            for (int s = 0; s < 8; ++s) {
-                double v = 0.0;
-                for (int a = 0; a < 3; ++a) v = __dadd_rn(v, ((s >> a) & 1) ? -d[a] : d[a]);
-                cost[k][s] = v;
-            }
+        const bool child = j < nch;
+        double d[3], cost[8];
+        for (int a = 0; a < 3; ++a)
+            d[a] = __dsub_rn(__dmul_rn(0.5, __dadd_rn(double(c.lo[a]), double(c.hi[a]))), double(cen(b.lo[a], b.hi[a])));
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            double v = 0.0;
+            for (int a = 0; a < 3; ++a) v = __dadd_rn(v, ((s >> a) & 1) ? -d[a] : d[a]);
+            cost[s] = v;
         }
-        int slot_of[8];
-        bool slot_used[8] = {false, false, false, false, false, false, false, false};
-        bool cdone[8] = {false, false, false, false, false, false, false, false};
-        for (int round = 0; round < nch; ++round) {
-            int bc = -1, bs = -1;
-            double bcost = 0.0;
-            for (int k = 0; k < nch; ++k) {
-                if (cdone[k]) continue;
-                for (int s = 0; s < 8; ++s) {
-                    if (slot_used[s]) continue;
-                    if (bc < 0 || cost[k][s] < bcost) {
-                        bcost = cost[k][s];
-                        bc = k;
+        unsigned used = 0;
+        int slot = -1;
+        const int rounds = __reduce_max_sync(FULL, nch);
+        for (int round = 0; round < rounds; ++round) {
+            double best = 0.0;
+            int bs = -1;
+            if (child && slot < 0) {
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    if (!((used >> s) & 1u) && (bs < 0 || cost[s] < best)) {
+                        best = cost[s];
                         bs = s;
                     }
+            }
+            int bk = bs >= 0 ? j : -1;
+            for (int off = 1; off < 8; off <<= 1) {
+                const double oc = __shfl_xor_sync(FULL, best, off);
+                const int ok = __shfl_xor_sync(FULL, bk, off), os = __shfl_xor_sync(FULL, bs, off);
+                if (ok >= 0 && (bk < 0 || oc < best || (oc == best && ok < bk))) {
+                    best = oc;
+                    bk = ok;
+                    bs = os;
                 }
             }
-            cdone[bc] = true;
-            slot_used[bs] = true;
-            slot_of[bc] = bs;
+            // one lane's answer for the group, whatever the comparisons did on values not ordered
+            bk = __shfl_sync(FULL, bk, g0);
+            bs = __shfl_sync(FULL, bs, g0);
+            if (bk >= 0) {
+                used |= 1u << bs;
+                if (j == bk) slot = bs;
+            }
         }
-        int at_slot[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
-        for (int k = 0; k < nch; ++k) at_slot[slot_of[k]] = ch[k];
+        if (!child) {  // the empty slots, in order
+            int k = j - nch;
+            for (int s = 0; s < 8; ++s)
+                if (!((used >> s) & 1u) && k-- == 0) slot = s;
+        }
         // quantisation (encode_node of the host builder)
-        BVH8Node N;
-        {
-            uint32_t* w = reinterpret_cast<uint32_t*>(&N);
-            for (int k = 0; k < 20; ++k) w[k] = 0;
-        }
         double mext = 0.0, mabs = 0.0;
         for (int a = 0; a < 3; ++a) {
             mext = fmax(mext, __dsub_rn(double(b.hi[a]), double(b.lo[a])));
             mabs = fmax(mabs, fmax(fabs(double(b.lo[a])), fabs(double(b.hi[a]))));
         }
         const double pad = __dadd_rn(__dadd_rn(__dmul_rn(1e-4, mext), __dmul_rn(1e-7, mabs)), 1e-30);
-        double hi_d[3];
+        BVH8Node& N = s_node[g];
         for (int a = 0; a < 3; ++a) {
             const double lo_d = __dsub_rn(double(b.lo[a]), pad);
-            hi_d[a] = __dadd_rn(double(b.hi[a]), pad);
+            const double hi_d = __dadd_rn(double(b.hi[a]), pad);
             float pf = __double2float_rn(lo_d);
             if (double(pf) > lo_d) pf = nextafterf(pf, -FLT_MAX);
-            N.p[a] = pf;
-        }
-        for (int a = 0; a < 3; ++a) {
-            const double ext = __dsub_rn(hi_d[a], double(N.p[a]));
+            const double ext = __dsub_rn(hi_d, double(pf));
             int e = -126;
             if (ext > 0.0) e = ceil_log2(__ddiv_rn(ext, 255.0));
             e = max(-126, min(127, e));
             while (ldexp(255.0, e) < ext && e < 127) ++e;
-            N.e[a] = uint8_t(e + 127);
+            uint8_t ql = 0xff, qh = 0x00;
+            if (child) {
+                const double scale = ldexp(1.0, e);
+                const double lq = floor(__dsub_rn(__ddiv_rn(__dsub_rn(double(c.lo[a]), double(pf)), scale), 0.01));
+                const double hq = ceil(__dadd_rn(__ddiv_rn(__dsub_rn(double(c.hi[a]), double(pf)), scale), 0.01));
+                ql = uint8_t(fmax(0.0, fmin(255.0, lq)));
+                qh = uint8_t(fmax(0.0, fmin(255.0, hq)));
+            }
+            (a == 0 ? N.qlox : a == 1 ? N.qloy : N.qloz)[slot] = ql;
+            (a == 0 ? N.qhix : a == 1 ? N.qhiy : N.qhiz)[slot] = qh;
+            if (j == 0) {
+                N.p[a] = pf;
+                N.e[a] = uint8_t(e + 127);
+            }
         }
-        uint8_t* qlo[3] = {N.qlox, N.qloy, N.qloz};
-        uint8_t* qhi[3] = {N.qhix, N.qhiy, N.qhiz};
-        for (int s = 0; s < 8; ++s) {
-            for (int a = 0; a < 3; ++a) {
-                if (at_slot[s] < 0) {
-                    qlo[a][s] = 0xff;
-                    qhi[a][s] = 0x00;
-                    continue;
+        const bool leaf = child && (c.left < 0 || c.count <= kMaxLeafPrims);
+        unsigned lm = leaf ? 1u << slot : 0u, im = child && !leaf ? 1u << slot : 0u;
+        for (int off = 1; off < 8; off <<= 1) {
+            lm |= __shfl_xor_sync(FULL, lm, off);
+            im |= __shfl_xor_sync(FULL, im, off);
+        }
+        const int ni = __popc(im), nl = __popc(lm);
+        if (j == 0) {
+            N.imask = uint8_t(im);
+            N.child_base = N.tri_base = 0u;
+            N.meta[0] = uint8_t(lm);
+            for (int k = 1; k < 8; ++k) N.meta[k] = 0;
+            s_count[g] = on ? (TileWord(nl) << 31 | TileWord(ni)) : 0;
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) {  // places of the tile's items
+            const TileWord mine = lane < kColItems ? s_count[lane] : 0;
+            TileWord incl = mine;
+            for (int off = 1; off < 32; off <<= 1) {
+                const TileWord v = __shfl_up_sync(FULL, incl, off);
+                if (lane >= off) incl += v;
+            }
+            const TileWord total = __shfl_sync(FULL, incl, 31);
+            volatile TileWord* own = words + tile;
+            if (lane == 0) *own = (tile == 0 ? kPrefix : kOwn) | total;
+            TileWord before = 0;
+            for (int t = tile - 1; t >= 0; t -= 32) {
+                TileWord v = kPrefix;
+                if (t - lane >= 0) {
+                    volatile const TileWord* p = words + (t - lane);
+                    v = *p;
+                    for (int polls = 0; !(v & (kOwn | kPrefix)) && polls < kPollLimit; ++polls) v = *p;
+                    if (!(v & (kOwn | kPrefix))) {
+                        *err = 1;
+                        v = kPrefix;
+                    }
                 }
-                const BinNode& c = bn[at_slot[s]];
-                const double scale = ldexp(1.0, int(N.e[a]) - 127);
-                const double l = floor(__dsub_rn(__ddiv_rn(__dsub_rn(double(c.lo[a]), double(N.p[a])), scale), 0.01));
-                const double h = ceil(__dadd_rn(__ddiv_rn(__dsub_rn(double(c.hi[a]), double(N.p[a])), scale), 0.01));
-                qlo[a][s] = uint8_t(fmax(0.0, fmin(255.0, l)));
-                qhi[a][s] = uint8_t(fmax(0.0, fmin(255.0, h)));
+                const unsigned done = __ballot_sync(FULL, (v & kPrefix) != 0);
+                const int stop = done ? __ffs(done) - 1 : 31;
+                TileWord x = lane <= stop ? (v & kCounts) : 0;
+                for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(FULL, x, off);
+                before += x;
+                if (done) break;
+            }
+            if (lane == 0 && tile) *own = kPrefix | (before + total);
+            if (lane < kColItems) s_count[lane] = before + incl - mine;
+            if (lane == 0 && tile == tiles - 1) {  // the next level
+                const long long start = (long long)o + n_items;
+                const long long n = (long long)((before + total) & kIntMask);
+                lvl[2 * (l + 1)] = int(start);
+                lvl[2 * (l + 1) + 1] = start + n > cap ? 0 : int(n);
+                if (start + n > cap) *err = 1;
             }
         }
-        int ni = 0, nl = 0;
-        for (int s = 0; s < 8; ++s) {
-            const int c = at_slot[s];
-            if (c < 0) continue;
-            const BinNode& cn = bn[c];
-            if (cn.left < 0 || cn.count <= kMaxLeafPrims) {
-                leaf_prim[size_t(it) * 8 + nl] = ord_fin[cn.begin];  // one primitive per leaf slot
-                ++nl;
-                N.meta[0] = uint8_t(N.meta[0] | (1u << s));
-            } else {
-                N.imask = uint8_t(N.imask | (1u << s));
-                child_bn[size_t(it) * 8 + ni] = c;
-                ++ni;
+        __syncthreads();
+        if (on) {
+            const int cs = int(s_count[g] & kIntMask), ls = int(s_count[g] >> 31);
+            const size_t at = size_t(o) + it;
+            if (leaf) leaf_prim_all[at * 8 + __popc(lm & ((1u << slot) - 1u))] = ord_fin[c.begin];
+            else if (child) {
+                const long long to = (long long)o + n_items + cs + __popc(im & ((1u << slot) - 1u));
+                if (to < cap) items_all[to] = Item{id, item.tree};
             }
+            if (j < 5) reinterpret_cast<uint4*>(tmp_all + at)[j] = reinterpret_cast<const uint4*>(&N)[j];
+            if (j == 5) n_leaf_all[at] = nl;
+            if (j == 6) cs_all[at] = cs;
+            if (j == 7) ls_all[at] = ls;
         }
-        tmp[it] = N;
-        n_int[it] = ni;
-        n_leaf[it] = nl;
+        __syncthreads();
     }
 }
 
-// next level: item cs[it] + k is internal child k of item it; the next level starts right
-// after this one
-__global__ void k_emit(Span sp, Item* items_all, const int* n_int_all, const int* cs_all, const int* child_bn_all,
-                       long long cap) {
-    const int o = sp.off(), n_items = sp.count();
-    const Item* items = items_all + o;
-    const int *n_int = n_int_all + o, *cs = cs_all + o;
-    const int* child_bn = child_bn_all + size_t(o) * 8;
-    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n_items; it += gridDim.x * blockDim.x)
-        for (int k = 0; k < n_int[it]; ++k) {
-            const long long at = (long long)o + n_items + cs[it] + k;  // past the capacity: k_level_next flags it
-            if (at < cap) items_all[at] = Item{child_bn[size_t(it) * 8 + k], items[it].tree};
+// The levels of the table in shared memory, for kernels over the items of all levels.
+struct Levels {
+    int off[kMaxLevels + 1];
+    int n;
+    __device__ void load(const int* lvl, int num_levels) {
+        for (int l = threadIdx.x; l <= num_levels; l += blockDim.x) off[l] = l < num_levels ? lvl[2 * l] : 0;
+        if (threadIdx.x == 0) {
+            // an empty level past the last has no offset of its own
+            int k = 1;
+            while (k < num_levels && lvl[2 * k + 1] > 0) ++k;
+            n = k;
         }
-}
+        __syncthreads();
+        if (threadIdx.x == 0) off[n] = lvl[2 * (n - 1)] + lvl[2 * (n - 1) + 1];
+        __syncthreads();
+    }
+    __device__ int total() const { return off[n]; }
+    __device__ int of(int at) const {
+        int lo = 0, hi = n - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (off[mid] <= at) lo = mid;
+            else hi = mid - 1;
+        }
+        return lo;
+    }
+};
 
-// Level l + 1 of the table: it starts after level l and holds *n_next items (the total of the
-// scan of level l's internal-child counts). Past the capacity it is left empty and err is set.
-__global__ void k_level_next(int* lvl, int l, const int* n_next, long long cap, int* err) {
-    const long long o = (long long)lvl[2 * l] + lvl[2 * l + 1];
-    const int n = *n_next;
-    lvl[2 * (l + 1)] = int(o);
-    if (o + n > cap) {
-        lvl[2 * (l + 1) + 1] = 0;
-        *err = 1;
-    } else {
-        lvl[2 * (l + 1) + 1] = n;
-    }
-}
-
-// exclusive scan of n ints (in -> out), total to *total; three passes over blocks of 1024
-constexpr int kScanBlock = 1024;
-__global__ void __launch_bounds__(256) k_scan_local(Span sp, const int* in_all, int* out_all, int* block_sums) {
-    __shared__ int sh[256];
-    const int o = sp.off(), n = sp.count();
-    const int* in = in_all + o;
-    int* out = out_all + o;
-    const int base = blockIdx.x * kScanBlock;
-    if (blockIdx.x > 0 && base >= n) return;  // block 0 always writes its (maybe empty) sum
-    int v[4], s = 0;
-    for (int k = 0; k < 4; ++k) {
-        const int i = base + int(threadIdx.x) * 4 + k;
-        v[k] = i < n ? in[i] : 0;
-        s += v[k];
-    }
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 1; off < 256; off <<= 1) {
-        const int t = threadIdx.x >= unsigned(off) ? sh[threadIdx.x - off] : 0;
-        __syncthreads();
-        sh[threadIdx.x] += t;
-        __syncthreads();
-    }
-    int run = sh[threadIdx.x] - s;
-    for (int k = 0; k < 4; ++k) {
-        const int i = base + int(threadIdx.x) * 4 + k;
-        if (i < n) out[i] = run;
-        run += v[k];
-    }
-    if (threadIdx.x == 255) block_sums[blockIdx.x] = sh[255];
-}
-__global__ void __launch_bounds__(1024) k_scan_sums(Span sp, int* block_sums, int* total) {
-    __shared__ int sh[1024];
-    const int nb = max(1, (sp.count() + kScanBlock - 1) / kScanBlock);
-    const int per = (nb + 1023) / 1024;
-    const int b0 = min(nb, int(threadIdx.x) * per), b1 = min(nb, b0 + per);
-    int s = 0;
-    for (int b = b0; b < b1; ++b) s += block_sums[b];
-    sh[threadIdx.x] = s;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const int t = threadIdx.x >= unsigned(off) ? sh[threadIdx.x - off] : 0;
-        __syncthreads();
-        sh[threadIdx.x] += t;
-        __syncthreads();
-    }
-    int run = sh[threadIdx.x] - s;
-    for (int b = b0; b < b1; ++b) {
-        const int v = block_sums[b];
-        block_sums[b] = run;
-        run += v;
-    }
-    if (threadIdx.x == 1023) *total = sh[1023];
-}
-__global__ void k_scan_add(Span sp, int* out_all, const int* block_sums) {
-    const int n = sp.count();
-    int* out = out_all + sp.off();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        out[i] += block_sums[i / kScanBlock];
-}
-
-// Where each tree's items of a level start and end: first[t] (atomic min) and last[t] (max).
-__global__ void k_bounds(const Item* items, int n_items, int* first, int* last) {
-    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n_items; it += gridDim.x * blockDim.x) {
-        const int t = items[it].tree;
-        if (it == 0 || items[it - 1].tree != t) first[t] = it;
-        if (it == n_items - 1 || items[it + 1].tree != t) last[t] = it;
+// Where each tree's items of each level start and end, from the level's start.
+__global__ void k_bounds(const int* lvl, int num_levels, const Item* items, int num_trees, int* first, int* last) {
+    __shared__ Levels V;
+    V.load(lvl, num_levels);
+    for (int at = blockIdx.x * blockDim.x + threadIdx.x; at < V.total(); at += gridDim.x * blockDim.x) {
+        const int L = V.of(at), it = at - V.off[L], n = V.off[L + 1] - V.off[L];
+        const int t = items[at].tree;
+        if (it == 0 || items[at - 1].tree != t) first[size_t(L) * num_trees + t] = it;
+        if (it == n - 1 || items[at + 1].tree != t) last[size_t(L) * num_trees + t] = it;
     }
 }
 
@@ -1039,7 +1316,7 @@ __global__ void k_bounds(const Item* items, int n_items, int* first, int* last) 
 // records relative to the tree), total nodes and depth. One thread per tree after a scan of the
 // trees' node totals (single block).
 __global__ void __launch_bounds__(1024) k_tree_offsets(int num_trees, int num_levels, const int* first, const int* last,
-                                                       const int* const* ls_level, const int* const* nl_level,
+                                                       const int* lvl, const int* ls, const int* n_leaf,
                                                        uint32_t node_base, uint32_t* node_off, uint32_t* leaf_off,
                                                        uint32_t* tree_nodes, int* tree_depth, uint32_t* tree_root) {
     __shared__ uint32_t part[1024];
@@ -1080,28 +1357,32 @@ __global__ void __launch_bounds__(1024) k_tree_offsets(int num_trees, int num_le
             const int l = last[size_t(L) * num_trees + t];
             if (l < f) continue;
             run += uint32_t(l - f + 1);
-            lrun += uint32_t(ls_level[L][l] + nl_level[L][l] - ls_level[L][f]);
+            const int o = lvl[2 * L];
+            lrun += uint32_t(ls[o + l] + n_leaf[o + l] - ls[o + f]);
         }
     }
 }
 
-// Final nodes of one level and their leaf records.
-__global__ void k_place(const Item* items, int n_items, int L, int num_trees, const BVH8Node* tmp, const int* cs,
-                        const int* ls, const int* n_leaf, const int* leaf_prim, const int* first,
+// Final nodes and their leaf records.
+__global__ void k_place(const int* lvl, int num_levels, const Item* items, int num_trees, const BVH8Node* tmp,
+                        const int* cs, const int* ls, const int* n_leaf, const int* leaf_prim, const int* first,
                         const uint32_t* node_off, const uint32_t* leaf_off, const int* tree_begin, bool global_tri,
-                        uint32_t node_base, uint32_t total_nodes, BVH8Node* nodes, uint32_t* leaf_out) {
-    for (int it = blockIdx.x * blockDim.x + threadIdx.x; it < n_items; it += gridDim.x * blockDim.x) {
-        const int t = items[it].tree;
+                        uint32_t node_base, uint32_t node_cap, BVH8Node* nodes, uint32_t* leaf_out) {
+    __shared__ Levels V;
+    V.load(lvl, num_levels);
+    for (int at = blockIdx.x * blockDim.x + threadIdx.x; at < V.total(); at += gridDim.x * blockDim.x) {
+        const int L = V.of(at), o = V.off[L];
+        const int t = items[at].tree;
         const int f = first[size_t(L) * num_trees + t];
-        const uint32_t idx = node_off[size_t(L) * num_trees + t] + uint32_t(it - f);
-        BVH8Node N = tmp[it];
-        N.child_base = node_off[size_t(L + 1) * num_trees + t] + uint32_t(cs[it] - cs[f]);
-        const uint32_t rec = leaf_off[size_t(L) * num_trees + t] + uint32_t(ls[it] - ls[f]);
+        const uint32_t idx = node_off[size_t(L) * num_trees + t] + uint32_t(at - o - f);
+        BVH8Node N = tmp[at];
+        N.child_base = node_off[size_t(L + 1) * num_trees + t] + uint32_t(cs[at] - cs[o + f]);
+        const uint32_t rec = leaf_off[size_t(L) * num_trees + t] + uint32_t(ls[at] - ls[o + f]);
         N.tri_base = rec + (global_tri ? uint32_t(tree_begin[t]) : 0u);
-        if (idx - node_base < total_nodes) nodes[idx - node_base] = N;
-        for (int k = 0; k < n_leaf[it]; ++k) {
+        if (idx - node_base < node_cap) nodes[idx - node_base] = N;
+        for (int k = 0; k < n_leaf[at]; ++k) {
             const size_t r = size_t(tree_begin[t]) + rec + k;
-            if (r < size_t(tree_begin[t + 1])) leaf_out[r] = uint32_t(leaf_prim[size_t(it) * 8 + k]);
+            if (r < size_t(tree_begin[t + 1])) leaf_out[r] = uint32_t(leaf_prim[size_t(at) * 8 + k]);
         }
     }
 }
@@ -1313,36 +1594,43 @@ __global__ void k_flat_records(const uint32_t* leaf_prim, int n, const int* flat
     }
 }
 
-// device buffers of one build, freed together
+// device buffers of one build, freed together: carved from one block of the expected size (an
+// allocation is a driver call of 30 to 100 us while other threads of a scene build make theirs)
 struct Bufs {
     cudaStream_t st;
     std::vector<void*> p;
-    explicit Bufs(cudaStream_t s) : st(s) {}
+    char* at = nullptr;
+    size_t left = 0;
+    Bufs(cudaStream_t s, size_t expected) : st(s) {
+        at = raw(expected);
+        left = at ? expected : 0;
+    }
+    Bufs(const Bufs&) = delete;
+    Bufs& operator=(const Bufs&) = delete;
     ~Bufs() {
         for (void* q : p) scratch_free(q, st);
     }
+    char* raw(size_t bytes) {
+        void* q = nullptr;
+        if (scratch_alloc(&q, bytes, st) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        p.push_back(q);
+        return static_cast<char*>(q);
+    }
     template <class T>
     T* get(size_t n) {
-        void* q = nullptr;
-        if (scratch_alloc(&q, std::max<size_t>(n, 1) * sizeof(T), st) != cudaSuccess) return nullptr;
-        p.push_back(q);
-        return static_cast<T*>(q);
+        const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~size_t(255);
+        if (bytes > left) return reinterpret_cast<T*>(raw(bytes));
+        T* q = reinterpret_cast<T*>(at);
+        at += bytes;
+        left -= bytes;
+        return q;
     }
 };
 
 int grid_for(int n, int per_block, int cap) { return std::max(1, std::min(cap, (n + per_block - 1) / per_block)); }
-
-// exclusive scan of n device ints (in -> out); the total lands in *total (device)
-// Exclusive scan of sp's items of in into out (both indexed from the level start); max_n bounds
-// the count for the launch shapes. The block sums need max(1, ceil(max_n / kScanBlock)) ints.
-int device_scan(Span sp, int max_n, const int* in, int* out, int* total, int* block_sums, cudaStream_t st) {
-    const int nb = std::max(1, (max_n + kScanBlock - 1) / kScanBlock);
-    k_scan_local<<<nb, 256, 0, st>>>(sp, in, out, block_sums);
-    k_scan_sums<<<1, 1024, 0, st>>>(sp, block_sums, total);
-    k_scan_add<<<grid_for(max_n, 256, 4096), 256, 0, st>>>(sp, out, block_sums);
-    LUX_CUDA(cudaGetLastError());
-    return LUX_OK;
-}
 
 }  // namespace
 
@@ -1354,241 +1642,218 @@ void DeviceBvh8::release() {
     num_nodes = 0;
 }
 
+namespace {
+
+// One build. levels: binary levels of large nodes that are launched; *unfinished is set when nodes
+// of more than kMedium primitives are left after them.
+//
+// Everything is enqueued without reading a size back: every kernel takes its level's counts from
+// the device (the two large lists alternate, binary ids continue from ctr[3], and a level past the
+// last has no nodes, so its kernels do nothing), buffers have room for the most there can be, and
+// one wait ends the build. Launches and read-backs in turn cost more than the kernels: while the
+// texture thread of a scene build copies from pageable memory, a driver call of this thread can
+// wait 1 to 3 ms (1M triangles: 4.0 ms of kernels took 7.3 ms with a read-back per stage, 5.9 so).
+int build_attempt(const float* d_boxes, const std::vector<int>& tree_begin, uint32_t node_base, bool global_tri,
+                  cudaStream_t st, int levels, DeviceBvh8& out, bool* unfinished) {
+    const int G = int(tree_begin.size()) - 1;
+    const int N = tree_begin[G];
+    const size_t bn_cap = size_t(2) * N;
+    const int large_cap = N / (kMedium + 1) + 1;
+    const int medium_cap = N / (kSmall + 1) + 1;
+    const int chunk_cap = large_cap + N / kChunk + 1;
+    const size_t item_cap = size_t(N) + G;
+    const size_t words_n = item_cap / kColItems + kMaxLevels + 2;
+    int max_tree = 1;
+    for (int t = 0; t < G; ++t) max_tree = std::max(max_tree, tree_begin[t + 1] - tree_begin[t]);
+    // 8-wide levels a tree of the largest size usually has (about one per three binary levels of a
+    // binary depth near 1.5 log2 n), and two more
+    const int wide0 = std::min(kMaxLevels, int(std::ceil(0.5 * std::log2(double(max_tree) + 1.0))) + 3);
+    const size_t expected = size_t(N) * (12 + 2 * sizeof(BinNode) + 4) + size_t(medium_cap) * 4 +
+                            size_t(large_cap) * (sizeof(Slot) + 8 + 3 * kBins * 28) + size_t(chunk_cap) * 16 +
+                            item_cap * (sizeof(Item) + sizeof(BVH8Node) + 12 + 32) + words_n * 8 +
+                            size_t(G) * (size_t(wide0) * 16 + 32) + 40 * 256 + 8192;
+    Bufs B(st, expected);
+    int* d_tb = B.get<int>(G + 1);
+    int* ord[2] = {B.get<int>(N), B.get<int>(N)};
+    int* ord_fin = B.get<int>(N);
+    BinNode* bn = B.get<BinNode>(bn_cap);
+    int* large[2] = {B.get<int>(large_cap), B.get<int>(large_cap)};
+    unsigned* medium = B.get<unsigned>(medium_cap);
+    int* small = B.get<int>(N / 2 + 1);
+    Slot* slots = B.get<Slot>(large_cap);
+    unsigned* bin_cnt = B.get<unsigned>(size_t(large_cap) * 3 * kBins);
+    unsigned* bin_lo = B.get<unsigned>(size_t(large_cap) * 3 * kBins * 3);
+    unsigned* bin_hi = B.get<unsigned>(size_t(large_cap) * 3 * kBins * 3);
+    int* chunk_slot = B.get<int>(chunk_cap);
+    int* chunk_start = B.get<int>(chunk_cap);
+    int* chunk_left = B.get<int>(chunk_cap);
+    int* chunk_lbase = B.get<int>(chunk_cap);
+    Item* items = B.get<Item>(item_cap);
+    BVH8Node* tmp = B.get<BVH8Node>(item_cap);
+    int* n_leaf = B.get<int>(item_cap);
+    int* cs = B.get<int>(item_cap);
+    int* ls = B.get<int>(item_cap);
+    int* leafp = B.get<int>(item_cap * 8);
+    // Words that start at zero, one block: ctr (0,1: large list sizes; 2: small list size; 3: next
+    // binary id; 4: chunks; 5: medium list size; 7: capacity error), the level table (offset and
+    // count per 8-wide level, then an error word), tile counters, look-back words.
+    constexpr int kLvl = 8, kErr = kLvl + 2 * kMaxLevels + 2, kTiles = kErr + 2, kWords = kTiles + kMaxLevels + 2;
+    static_assert(kWords % 2 == 0, "look-back words are 8 bytes");
+    const size_t zero_n = size_t(kWords) + 2 * words_n;
+    int* zero = B.get<int>(zero_n);
+    if (!d_tb || !ord[0] || !ord[1] || !ord_fin || !bn || !large[0] || !large[1] || !medium || !small || !slots ||
+        !bin_cnt || !bin_lo || !bin_hi || !chunk_slot || !chunk_start || !chunk_left || !chunk_lbase || !items || !tmp ||
+        !n_leaf || !cs || !ls || !leafp || !zero)
+        return fail(LUX_ERR_OOM, "BVH build: device scratch allocation failed");
+    int *ctr = zero, *lvl = zero + kLvl, *err = zero + kErr, *tile_ctr = zero + kTiles;
+    TileWord* words = reinterpret_cast<TileWord*>(zero + kWords);
+    out.stream = st;
+    if (scratch_alloc(reinterpret_cast<void**>(&out.nodes), sizeof(BVH8Node) * item_cap, st) != cudaSuccess ||
+        scratch_alloc(reinterpret_cast<void**>(&out.leaf_prim), sizeof(uint32_t) * size_t(N), st) != cudaSuccess) {
+        cudaGetLastError();
+        out.release();
+        return fail(LUX_ERR_OOM, "BVH build: node allocation failed");
+    }
+    // page-locked: tree starts, roots and the start of the level table go up, the tables and the
+    // trees' results come down
+    const size_t host_n = size_t(kTiles) + size_t(G + 1) + 2 * size_t(G) + 3 * size_t(G) + 8;
+    struct HostBlock {  // back to the pool once no copy can still use it
+        int* p;
+        size_t bytes;
+        cudaStream_t st;
+        ~HostBlock() {
+            cudaStreamSynchronize(st);
+            pinned_put(p, bytes);
+        }
+    } hb{static_cast<int*>(pinned_get(host_n * sizeof(int))), host_n * sizeof(int), st};
+    if (!hb.p) return fail(LUX_ERR_OOM, "BVH build: page-locked host allocation failed");
+    int* h_zero = hb.p;
+    int* h_tb = h_zero + kTiles;
+    Item* h_roots = reinterpret_cast<Item*>(h_tb + G + 1);
+    int* h_out = h_tb + G + 1 + 2 * G;
+    std::memcpy(h_tb, tree_begin.data(), sizeof(int) * (G + 1));
+    for (int t = 0; t < G; ++t) h_roots[t] = Item{t, t};
+    std::memset(h_zero, 0, sizeof(int) * kTiles);
+    h_zero[3] = G;          // binary ids after the roots'
+    h_zero[kLvl + 1] = G;   // level 0: the roots
+    LUX_CUDA(cudaMemcpyAsync(d_tb, h_tb, sizeof(int) * (G + 1), cudaMemcpyHostToDevice, st));
+    LUX_CUDA(cudaMemcpyAsync(items, h_roots, sizeof(Item) * G, cudaMemcpyHostToDevice, st));
+    LUX_CUDA(cudaMemsetAsync(zero, 0, sizeof(int) * zero_n, st));
+    LUX_CUDA(cudaMemcpyAsync(zero, h_zero, sizeof(int) * kTiles, cudaMemcpyHostToDevice, st));
+    // every index array starts in range, so no read can leave its buffer whatever is computed
+    LUX_CUDA(cudaMemsetAsync(ord[1], 0, sizeof(int) * size_t(N), st));
+    LUX_CUDA(cudaMemsetAsync(ord_fin, 0, sizeof(int) * size_t(N), st));
+    LUX_CUDA(cudaMemsetAsync(bn, 0, sizeof(BinNode) * bn_cap, st));
+    LUX_CUDA(cudaMemsetAsync(out.leaf_prim, 0, sizeof(uint32_t) * size_t(N), st));
+    k_iota<<<grid_for(N, 256, 4096), 256, 0, st>>>(ord[0], N);
+    k_roots<<<grid_for(G, 128, 1024), 128, 0, st>>>(d_boxes, d_tb, G, bn, ord[0], ord_fin, large[0], ctr + 0, medium,
+                                                   ctr + 5, small, ctr + 2);
+    // ---- binary levels of large nodes ----
+    const int grid_s = grid_for(large_cap, 128, 4096);
+    const int grid_sp = grid_for(large_cap, kSplitWarps, 4096);
+    const int grid_clear = grid_for(large_cap * 3 * kBins, 256, 148 * 16);
+    const int grid_c = std::min(chunk_cap, 148 * 8);
+    int cur = 0;
+    for (int b = 0; b < levels; ++b) {
+        const int nxt = cur ^ 1;
+        k_chunks<<<1, 1024, 0, st>>>(large[cur], ctr + cur, bn, slots, chunk_slot, chunk_start, ctr + 4);
+        k_bin_clear<<<grid_clear, 256, 0, st>>>(ctr + cur, bin_cnt, bin_lo, bin_hi);
+        k_reduce<<<grid_c, kBlock, 0, st>>>(d_boxes, ord[cur], large[cur], bn, slots, chunk_slot, chunk_start, ctr + 4);
+        k_bin_setup<<<grid_s, 128, 0, st>>>(large[cur], ctr + cur, bn, slots);
+        k_bin<<<grid_c, kBlock, 0, st>>>(d_boxes, ord[cur], large[cur], bn, slots, chunk_slot, chunk_start, ctr + 4,
+                                          bin_cnt, bin_lo, bin_hi);
+        k_split<<<grid_sp, 32 * kSplitWarps, 0, st>>>(large[cur], ctr + cur, bn, slots, bin_cnt, bin_lo, bin_hi);
+        k_count_left<<<grid_c, kBlock, 0, st>>>(d_boxes, ord[cur], large[cur], bn, slots, chunk_slot, chunk_start,
+                                                 ctr + 4, chunk_left);
+        k_chunk_base<<<grid_s, 128, 0, st>>>(ctr + cur, slots, chunk_left, chunk_lbase);
+        k_scatter<<<grid_c, kBlock, 0, st>>>(d_boxes, ord[cur], ord[nxt], large[cur], bn, slots, chunk_slot,
+                                              chunk_start, ctr + 4, chunk_lbase);
+        k_children<<<grid_s, 128, 0, st>>>(d_boxes, ord[nxt], ord_fin, large[cur], ctr + cur, bn, slots, ctr + 3,
+                                           int(bn_cap), ctr + 7, large[nxt], ctr + nxt, medium, ctr + 5,
+                                           unsigned(nxt), small, ctr + 2);
+        k_level_advance<<<1, 1, 0, st>>>(ctr + cur, ctr + 3);
+        LUX_CUDA(cudaGetLastError());
+        cur = nxt;
+    }
+    // ---- medium and small subtrees, from the lists' device counts: binary ids continue in ctr[3] ----
+    k_medium<<<grid_for(medium_cap, 1, 148 * 7), kBlock, 0, st>>>(d_boxes, ord[0], ord[1], medium, ctr + 5, bn, int(bn_cap),
+                                                                  ctr + 3, ctr + 7, ord_fin, small, ctr + 2);
+    k_small<<<grid_for(N / 2 + 1, kSmallWarps, 148 * 16), 32 * kSmallWarps, 0, st>>>(d_boxes, small, ctr + 2, bn, ord_fin,
+                                                                                     ctr + 3);
+    LUX_CUDA(cudaGetLastError());
+    // ---- collapse level by level, then the placement over all levels ----
+    const int grid_items = grid_for(int(item_cap), kColItems, 148 * 4);
+    const int grid_place = grid_for(int(item_cap), 128, 148 * 16);
+    int launched = 0, batch = wide0;
+    while (true) {
+        for (int l = launched; l < launched + batch; ++l)
+            k_collapse<<<grid_items, kColThreads, 0, st>>>(lvl, l, items, bn, ord_fin, tmp, n_leaf, cs, ls, leafp, words,
+                                                           tile_ctr, (long long)item_cap, err);
+        launched += batch;
+        const size_t lg = size_t(launched) * G;
+        int* first = B.get<int>(2 * lg);
+        uint32_t* node_off = B.get<uint32_t>(2 * (lg + G));
+        uint32_t* tree_out = B.get<uint32_t>(3 * size_t(G));  // roots, node counts, depths
+        if (!first || !node_off || !tree_out) return fail(LUX_ERR_OOM, "BVH build: device scratch allocation failed");
+        int* last = first + lg;
+        uint32_t* leaf_off = node_off + lg + G;
+        LUX_CUDA(cudaMemsetAsync(first, 0xff, 2 * sizeof(int) * lg, st));
+        k_bounds<<<grid_place, 128, 0, st>>>(lvl, launched, items, G, first, last);
+        k_tree_offsets<<<1, 1024, 0, st>>>(G, launched, first, last, lvl, ls, n_leaf, node_base, node_off, leaf_off,
+                                           tree_out + G, reinterpret_cast<int*>(tree_out + 2 * G), tree_out);
+        k_place<<<grid_place, 128, 0, st>>>(lvl, launched, items, G, tmp, cs, ls, n_leaf, leafp, first, node_off, leaf_off,
+                                            d_tb, global_tri, node_base, uint32_t(item_cap), out.nodes, out.leaf_prim);
+        LUX_CUDA(cudaGetLastError());
+        LUX_CUDA(cudaMemcpyAsync(h_zero, zero, sizeof(int) * kTiles, cudaMemcpyDeviceToHost, st));
+        LUX_CUDA(cudaMemcpyAsync(h_out, tree_out, 3 * sizeof(uint32_t) * G, cudaMemcpyDeviceToHost, st));
+        LUX_CUDA(cudaStreamSynchronize(st));
+        if (h_zero[7]) return fail(LUX_ERR_UNSUPPORTED, "BVH build: binary node capacity");
+        if (h_zero[cur]) {
+            *unfinished = true;
+            return LUX_OK;
+        }
+        if (h_zero[kErr]) return fail(LUX_ERR_UNSUPPORTED, "BVH build: 8-wide node capacity");
+        if (h_zero[kLvl + 2 * launched + 1] == 0) break;  // no level after the launched ones
+        batch = std::min(8, kMaxLevels - launched);
+        if (batch <= 0) return fail(LUX_ERR_UNSUPPORTED, "BVH build: too many 8-wide levels");
+    }
+    uint32_t total = 0;
+    for (int l = 0; l < launched; ++l) total += uint32_t(h_zero[kLvl + 2 * l + 1]);
+    out.root.assign(reinterpret_cast<uint32_t*>(h_out), reinterpret_cast<uint32_t*>(h_out) + G);
+    out.count.assign(reinterpret_cast<uint32_t*>(h_out) + G, reinterpret_cast<uint32_t*>(h_out) + 2 * G);
+    out.depth.assign(h_out + 2 * G, h_out + 3 * G);
+    out.num_nodes = total;
+    *unfinished = false;
+    return LUX_OK;
+}
+
+}  // namespace
+
 int build_bvh8_device(const float* d_boxes, const std::vector<int>& tree_begin, uint32_t node_base, bool global_tri,
                       cudaStream_t st, DeviceBvh8& out) {
     out.release();
     const int G = int(tree_begin.size()) - 1;
     if (G <= 0) return fail(LUX_ERR_INVALID, "BVH build without trees");
-    for (int t = 0; t < G; ++t)
-        if (tree_begin[t + 1] <= tree_begin[t]) return fail(LUX_ERR_INVALID, "BVH build: a tree without primitives");
-    const int N = tree_begin[G];
-    Bufs B(st);
-    int* d_tb = B.get<int>(G + 1);
-    int* ord[2] = {B.get<int>(N), B.get<int>(N)};
-    int* ord_fin = B.get<int>(N);
-    const size_t bn_cap = size_t(2) * N;
-    BinNode* bn = B.get<BinNode>(bn_cap);
-    const int large_cap = N / (kSmall + 1) + 1;
-    int* large[2] = {B.get<int>(large_cap), B.get<int>(large_cap)};
-    int* small = B.get<int>(N / 2 + 1);
-    int* ctr = B.get<int>(8);  // 0,1: large list sizes; 2: small list size; 3: next binary id; 4: chunks
-    Slot* slots = B.get<Slot>(large_cap);
-    unsigned* bin_cnt = B.get<unsigned>(size_t(large_cap) * 3 * kBins);
-    unsigned* bin_lo = B.get<unsigned>(size_t(large_cap) * 3 * kBins * 3);
-    unsigned* bin_hi = B.get<unsigned>(size_t(large_cap) * 3 * kBins * 3);
-    const int chunk_cap = large_cap + N / kChunk + 1;
-    int* chunk_slot = B.get<int>(chunk_cap);
-    int* chunk_start = B.get<int>(chunk_cap);
-    int* chunk_left = B.get<int>(chunk_cap);
-    int* chunk_lbase = B.get<int>(chunk_cap);
-    int* h_ctr = nullptr;
-    if (!d_tb || !ord[0] || !ord[1] || !ord_fin || !bn || !large[0] || !large[1] || !small || !ctr || !slots ||
-        !bin_cnt || !bin_lo || !bin_hi || !chunk_slot || !chunk_start || !chunk_left || !chunk_lbase)
-        return fail(LUX_ERR_OOM, "BVH build: device scratch allocation failed");
-    h_ctr = static_cast<int*>(pinned_get(8 * sizeof(int)));
-    if (!h_ctr) return fail(LUX_ERR_OOM, "BVH build: page-locked host allocation failed");
-    struct HostFree {  // back to the pool once no copy into it can still be queued
-        int* p;
-        cudaStream_t st;
-        ~HostFree() {
-            cudaStreamSynchronize(st);
-            pinned_put(p, 8 * sizeof(int));
-        }
-    } hf{h_ctr, st};
-    LUX_CUDA(cudaMemcpyAsync(d_tb, tree_begin.data(), sizeof(int) * (G + 1), cudaMemcpyHostToDevice, st));
-    LUX_CUDA(cudaMemsetAsync(ctr, 0, 8 * sizeof(int), st));
-    // every index array starts in range, so no read can leave its buffer whatever is computed
-    LUX_CUDA(cudaMemsetAsync(ord[1], 0, sizeof(int) * size_t(N), st));
-    LUX_CUDA(cudaMemsetAsync(ord_fin, 0, sizeof(int) * size_t(N), st));
-    LUX_CUDA(cudaMemsetAsync(bn, 0, sizeof(BinNode) * bn_cap, st));
-    k_iota<<<grid_for(N, 256, 4096), 256, 0, st>>>(ord[0], N);
-    k_roots<<<grid_for(G, 128, 1024), 128, 0, st>>>(d_boxes, d_tb, G, bn, ord[0], ord_fin, large[0], ctr + 0, small,
-                                                   ctr + 2);
-    LUX_CUDA(cudaGetLastError());
-    LUX_CUDA(cudaMemcpyAsync(h_ctr, ctr, 8 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    LUX_CUDA(cudaStreamSynchronize(st));
-    // Binary levels of large nodes, launched in batches without reading their sizes back:
-    // every kernel takes the level's node count from ctr[cur] (the two large lists alternate),
-    // binary ids continue from ctr[3], and a level past the last has no nodes, so its kernels
-    // do nothing. One read-back per batch finds the first empty level; ctr[7] flags a binary
-    // node table too small.
-    h_ctr[3] = G;
-    LUX_CUDA(cudaMemcpyAsync(ctr + 3, h_ctr + 3, sizeof(int), cudaMemcpyHostToDevice, st));
     int max_tree = 1;
-    for (int t = 0; t < G; ++t) max_tree = std::max(max_tree, tree_begin[t + 1] - tree_begin[t]);
-    const int grid_s = grid_for(large_cap, 128, 4096);
-    const int grid_sp = grid_for(large_cap, kSplitWarps, 4096);
-    const int grid_clear = grid_for(large_cap * 3 * kBins, 256, 148 * 16);
-    const int grid_c = std::min(chunk_cap, 148 * 8);
-    int cur = 0, levels = 0;
-    int batch = int(std::ceil(std::log2(double(max_tree) / double(kSmall) + 1.0))) + 2;
+    for (int t = 0; t < G; ++t) {
+        if (tree_begin[t + 1] <= tree_begin[t]) return fail(LUX_ERR_INVALID, "BVH build: a tree without primitives");
+        max_tree = std::max(max_tree, tree_begin[t + 1] - tree_begin[t]);
+    }
+    // Halving reaches kMedium in log2(max_tree / kMedium) levels; SAH splits of real scenes take a
+    // few more (16 instead of 10 for 1M triangles). Primitives that peel off a few at a time can take
+    // any number: the build is then repeated with four times the levels.
+    int levels = max_tree <= kMedium ? 0 : int(std::ceil(std::log2(double(max_tree) / kMedium))) + 8;
     while (true) {
-        for (int b = 0; b < batch; ++b) {
-            if (++levels > 4 * 64 + N) return fail(LUX_ERR_UNSUPPORTED, "BVH build did not converge");
-            const int nxt = cur ^ 1;
-            k_chunks<<<1, 1024, 0, st>>>(large[cur], ctr + cur, bn, slots, chunk_slot, chunk_start, ctr + 4);
-            k_bin_clear<<<grid_clear, 256, 0, st>>>(ctr + cur, bin_cnt, bin_lo, bin_hi);
-            k_reduce<<<grid_c, kBlock, 0, st>>>(d_boxes, ord[cur], large[cur], bn, slots, chunk_slot, chunk_start,
-                                                ctr + 4);
-            k_bin_setup<<<grid_s, 128, 0, st>>>(large[cur], ctr + cur, bn, slots);
-            k_bin<<<grid_c, kBlock, 0, st>>>(d_boxes, ord[cur], large[cur], bn, slots, chunk_slot, chunk_start, ctr + 4,
-                                              bin_cnt, bin_lo, bin_hi);
-            k_split<<<grid_sp, 32 * kSplitWarps, 0, st>>>(large[cur], ctr + cur, bn, slots, bin_cnt, bin_lo, bin_hi);
-            k_count_left<<<grid_c, kBlock, 0, st>>>(d_boxes, ord[cur], large[cur], bn, slots, chunk_slot, chunk_start,
-                                                     ctr + 4, chunk_left);
-            k_chunk_base<<<grid_s, 128, 0, st>>>(ctr + cur, slots, chunk_left, chunk_lbase);
-            k_scatter<<<grid_c, kBlock, 0, st>>>(d_boxes, ord[cur], ord[nxt], large[cur], bn, slots, chunk_slot,
-                                                  chunk_start, ctr + 4, chunk_lbase);
-            k_children<<<grid_s, 128, 0, st>>>(d_boxes, ord[nxt], ord_fin, large[cur], ctr + cur, bn, slots, ctr + 3,
-                                               int(bn_cap), ctr + 7, large[nxt], ctr + nxt, small, ctr + 2);
-            k_level_advance<<<1, 1, 0, st>>>(ctr + cur, ctr + 3);
-            LUX_CUDA(cudaGetLastError());
-            cur = nxt;
+        bool unfinished = false;
+        if (int rc = build_attempt(d_boxes, tree_begin, node_base, global_tri, st, levels, out, &unfinished)) {
+            out.release();
+            return rc;
         }
-        LUX_CUDA(cudaMemcpyAsync(h_ctr, ctr, 8 * sizeof(int), cudaMemcpyDeviceToHost, st));
-        LUX_CUDA(cudaStreamSynchronize(st));
-        if (h_ctr[7]) return fail(LUX_ERR_UNSUPPORTED, "BVH build: binary node capacity");
-        if (h_ctr[cur] == 0) break;
-        batch = 4;
-    }
-    // small subtrees: binary ids continue after the large levels' children
-    const int n_small = h_ctr[2];
-    if (n_small > 0) {
-        int* nid = ctr + 3;  // the next binary id, past every large level's children
-        k_small<<<grid_for(n_small, kSmallWarps, 148 * 16), 32 * kSmallWarps, 0, st>>>(d_boxes, small, ctr + 2, bn,
-                                                                                        ord_fin, nid);
-        LUX_CUDA(cudaGetLastError());
-    }
-
-    // ---- collapse, level by level ----
-    const size_t item_cap = size_t(N) + G;
-    Item* items = B.get<Item>(item_cap);
-    BVH8Node* tmp = B.get<BVH8Node>(item_cap);
-    int* n_int = B.get<int>(item_cap);
-    int* n_leaf = B.get<int>(item_cap);
-    int* cs = B.get<int>(item_cap);
-    int* ls = B.get<int>(item_cap);
-    int* child_bn = B.get<int>(item_cap * 8);
-    int* leafp = B.get<int>(item_cap * 8);
-    int* block_sums = B.get<int>(item_cap / kScanBlock + 2);
-    if (!items || !tmp || !n_int || !n_leaf || !cs || !ls || !child_bn || !leafp || !block_sums)
-        return fail(LUX_ERR_OOM, "BVH build: device scratch allocation failed");
-    {
-        std::vector<Item> roots(G);
-        for (int t = 0; t < G; ++t) roots[t] = Item{t, t};
-        LUX_CUDA(cudaMemcpyAsync(items, roots.data(), sizeof(Item) * G, cudaMemcpyHostToDevice, st));
-    }
-    // The levels are launched in batches without reading their sizes back: every kernel takes
-    // its level's offset and count from the device level table (lvl: offset, count per level;
-    // then an error word), and a level past the last is empty, so its kernels do nothing. One
-    // read-back of the table per batch finds the first empty level. The first batch covers the
-    // levels a tree of the largest size usually has (about one 8-wide level per three binary
-    // levels of a binary depth near 1.5 log2 n).
-    constexpr int kMaxLevels = 120;
-    int* lvl = B.get<int>(2 * kMaxLevels + 4);
-    int* h_lvl = static_cast<int*>(pinned_get(sizeof(int) * (2 * kMaxLevels + 4)));
-    struct LevelFree {
-        int* p;
-        cudaStream_t st;
-        ~LevelFree() {
-            cudaStreamSynchronize(st);
-            pinned_put(p, sizeof(int) * (2 * kMaxLevels + 4));
-        }
-    } lf{h_lvl, st};
-    if (!lvl || !h_lvl) return fail(LUX_ERR_OOM, "BVH build: level table allocation failed");
-    int* lvl_err = lvl + 2 * kMaxLevels + 2;
-    LUX_CUDA(cudaMemsetAsync(lvl, 0, sizeof(int) * (2 * kMaxLevels + 4), st));
-    {
-        const int first[2] = {0, G};
-        LUX_CUDA(cudaMemcpyAsync(lvl, first, sizeof(first), cudaMemcpyHostToDevice, st));
-        LUX_CUDA(cudaStreamSynchronize(st));  // `first` lives on this stack frame
-    }
-    const int max_n = int(item_cap);
-    const int grid_items = grid_for(max_n, 128, 148 * 16);
-    int launched = 0, L = -1;
-    batch = int(std::ceil(0.5 * std::log2(double(max_tree) + 1.0))) + 1;
-    while (L < 0) {
-        batch = std::min(batch, kMaxLevels - launched);
-        if (batch <= 0) return fail(LUX_ERR_UNSUPPORTED, "BVH build: too many 8-wide levels");
-        for (int l = launched; l < launched + batch; ++l) {
-            const Span sp{lvl, l, 0};
-            k_collapse<<<grid_items, 128, 0, st>>>(sp, items, bn, ord_fin, tmp, n_int, n_leaf, child_bn, leafp);
-            LUX_CUDA(cudaGetLastError());
-            if (int rc = device_scan(sp, max_n, n_leaf, ls, ctr + 5, block_sums, st)) return rc;
-            if (int rc = device_scan(sp, max_n, n_int, cs, ctr + 6, block_sums, st)) return rc;
-            k_level_next<<<1, 1, 0, st>>>(lvl, l, ctr + 6, (long long)item_cap, lvl_err);
-            k_emit<<<grid_items, 128, 0, st>>>(sp, items, n_int, cs, child_bn, (long long)item_cap);
-            LUX_CUDA(cudaGetLastError());
-        }
-        launched += batch;
-        LUX_CUDA(cudaMemcpyAsync(h_lvl, lvl, sizeof(int) * (2 * kMaxLevels + 4), cudaMemcpyDeviceToHost, st));
-        LUX_CUDA(cudaStreamSynchronize(st));
-        if (h_lvl[2 * kMaxLevels + 2]) return fail(LUX_ERR_UNSUPPORTED, "BVH build: 8-wide node capacity");
-        for (int l = 1; l <= launched; ++l)
-            if (h_lvl[2 * l + 1] == 0) {
-                L = l;
-                break;
-            }
-        batch = 3;
-    }
-    std::vector<size_t> lvl_off(L);
-    std::vector<int> lvl_n(L);
-    for (int l = 0; l < L; ++l) {
-        lvl_off[l] = size_t(h_lvl[2 * l]);
-        lvl_n[l] = h_lvl[2 * l + 1];
-    }
-    const size_t total_items = lvl_off.back() + size_t(lvl_n.back());
-
-    // ---- placement ----
-    int* first = B.get<int>(size_t(L) * G);
-    int* last = B.get<int>(size_t(L) * G);
-    uint32_t* node_off = B.get<uint32_t>(size_t(L + 1) * G);
-    uint32_t* leaf_off = B.get<uint32_t>(size_t(L + 1) * G);
-    uint32_t* tree_nodes = B.get<uint32_t>(G);
-    int* tree_depth = B.get<int>(G);
-    uint32_t* tree_root = B.get<uint32_t>(G);
-    const int** lsp = B.get<const int*>(L);
-    const int** nlp = B.get<const int*>(L);
-    if (!first || !last || !node_off || !leaf_off || !tree_nodes || !tree_depth || !tree_root || !lsp || !nlp)
-        return fail(LUX_ERR_OOM, "BVH build: device scratch allocation failed");
-    LUX_CUDA(cudaMemsetAsync(first, 0xff, sizeof(int) * size_t(L) * G, st));
-    LUX_CUDA(cudaMemsetAsync(last, 0xff, sizeof(int) * size_t(L) * G, st));
-    std::vector<const int*> h_lsp(L), h_nlp(L);
-    for (int l = 0; l < L; ++l) {
-        h_lsp[l] = ls + lvl_off[l];
-        h_nlp[l] = n_leaf + lvl_off[l];
-        k_bounds<<<grid_for(lvl_n[l], 128, 4096), 128, 0, st>>>(items + lvl_off[l], lvl_n[l], first + size_t(l) * G,
-                                                               last + size_t(l) * G);
-    }
-    LUX_CUDA(cudaMemcpyAsync(lsp, h_lsp.data(), sizeof(int*) * L, cudaMemcpyHostToDevice, st));
-    LUX_CUDA(cudaMemcpyAsync(nlp, h_nlp.data(), sizeof(int*) * L, cudaMemcpyHostToDevice, st));
-    k_tree_offsets<<<1, 1024, 0, st>>>(G, L, first, last, lsp, nlp, node_base, node_off, leaf_off, tree_nodes,
-                                       tree_depth, tree_root);
-    LUX_CUDA(cudaGetLastError());
-    out.stream = st;
-    if (scratch_alloc(reinterpret_cast<void**>(&out.nodes), sizeof(BVH8Node) * std::max<size_t>(total_items, 1), st) !=
-            cudaSuccess ||
-        scratch_alloc(reinterpret_cast<void**>(&out.leaf_prim), sizeof(uint32_t) * size_t(N), st) != cudaSuccess) {
+        if (!unfinished) return LUX_OK;
         out.release();
-        return fail(LUX_ERR_OOM, "BVH build: node allocation failed");
+        if (levels > 4 * (64 + max_tree / kMedium)) return fail(LUX_ERR_UNSUPPORTED, "BVH build did not converge");
+        levels *= 4;
     }
-    LUX_CUDA(cudaMemsetAsync(out.leaf_prim, 0, sizeof(uint32_t) * size_t(N), st));
-    for (int l = 0; l < L; ++l)
-        k_place<<<grid_for(lvl_n[l], 128, 4096), 128, 0, st>>>(items + lvl_off[l], lvl_n[l], l, G, tmp + lvl_off[l],
-                                                              cs + lvl_off[l], ls + lvl_off[l], n_leaf + lvl_off[l],
-                                                              leafp + lvl_off[l] * 8, first, node_off, leaf_off, d_tb,
-                                                              global_tri, node_base, uint32_t(total_items), out.nodes,
-                                                              out.leaf_prim);
-    LUX_CUDA(cudaGetLastError());
-    out.root.resize(G);
-    out.count.resize(G);
-    out.depth.resize(G);
-    LUX_CUDA(cudaMemcpyAsync(out.root.data(), tree_root, sizeof(uint32_t) * G, cudaMemcpyDeviceToHost, st));
-    LUX_CUDA(cudaMemcpyAsync(out.count.data(), tree_nodes, sizeof(uint32_t) * G, cudaMemcpyDeviceToHost, st));
-    LUX_CUDA(cudaMemcpyAsync(out.depth.data(), tree_depth, sizeof(int) * G, cudaMemcpyDeviceToHost, st));
-    LUX_CUDA(cudaStreamSynchronize(st));
-    out.num_nodes = uint32_t(total_items);
-    return LUX_OK;
 }
 
 cudaError_t launch_fill_mesh_ids(const uint32_t* tri_off, int num_meshes, int* prim_mesh, cudaStream_t st) {

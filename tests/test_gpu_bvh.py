@@ -66,3 +66,32 @@ def test_device_build_equals_host_build_on_scene_triangles():
         sizes.append(md.num_tris)
     tb = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
     same_build(np.concatenate(all_boxes), tb)
+
+
+@pytest.mark.parametrize("sizes,clustered,seed", [
+    ([1023, 1024, 1025], False, 6),         # around the largest subtree one block builds
+    ([1024] * 20, True, 7),
+    ([2049, 33, 2048, 1], True, 8),
+    ([300000], True, 9),
+])
+def test_block_subtrees_equal_host_build(sizes, clustered, seed):
+    tb = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    same_build(random_boxes(int(tb[-1]), seed=seed, clustered=clustered), tb)
+
+
+def test_lopsided_tree_equals_host_build():
+    """Groups of boxes at geometrically shrinking distances: each split takes off a group or two, so
+    the nodes above the block size take far more levels than halving would."""
+    g = np.random.default_rng(3)
+    lo = []
+    for k in range(60):
+        lo.append(2.0 ** (-2 * k) * (1.0 + 0.1 * g.random((60, 3))))
+    lo.append(2.0 ** -120 * g.random((1500, 3)))
+    lo = np.concatenate(lo).astype(np.float32)
+    boxes = np.concatenate([lo, lo * np.float32(1.01)], 1)[g.permutation(len(lo))]
+    same_build(np.ascontiguousarray(boxes), np.array([0, len(boxes)], np.int32))
+
+
+def test_coincident_boxes_equal_host_build():
+    one = np.array([[0.0, 0.0, 0.0, 1.0, 1.0, 1.0]], np.float32)
+    same_build(np.repeat(one, 5000, 0), np.array([0, 5000], np.int32))
