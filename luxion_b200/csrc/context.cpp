@@ -831,21 +831,6 @@ int alloc_wave(lux_ctx* C, int max_paths, int lanes) {
 bool whole_paths(const lux_ctx* C) {
     return !C->opt.ray_sorting && !C->opt.debug_bvh && !C->dopt.material_debug && !C->timing;
 }
-// Waves of at most kWholePerLane paths per lane of the whole-path kernel's grid (284k on 148 SMs)
-// run in it from the camera on. Above, the wavefront's full warps win: 0.81 against 1.18 ms for
-// 228k paths (477k triangles) and 0.35 against 0.53 for 66k (Cornell box), but 1.65 against 1.12 ms
-// for 367k (842k triangles). A larger wave hands over before one of the bounces 1 to kTailLast once
-// at most kTailPerLane paths per lane are left (114k) and two bounces or more are to come: a frame
-// of 2.07M paths, 1M triangles, depth 12 takes 4.18 ms instead of 5.34, while handing over at
-// twice that many took 5 to 20 % longer in 700k-triangle scenes. An attempt that finds more paths
-// left costs an empty launch.
-constexpr int kWholePerLane = 5;
-constexpr int kTailPerLane = 2;
-constexpr int kTailLast = 3;
-int path_limit(int per_lane) { return per_lane * path_grid_blocks() * kPathBlock; }
-int tail_attempts(int depth) { return std::max(0, std::min(kTailLast, depth - 2)); }
-bool try_tail(int bounce, int depth) { return bounce >= 1 && bounce <= kTailLast && bounce + 2 <= depth; }
-
 // Launches of one wave of n paths (enqueue_wave) added to the call's statistics.
 void count_launches(lux_ctx* C, int n) {
     const int depth = C->dopt.trace_depth;

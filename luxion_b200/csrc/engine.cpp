@@ -169,6 +169,9 @@ int enqueue_wave(lux_engine* E, int depth, int wave_paths, int trace_grid) {
     LUX_CUDA(cudaMemsetAsync(E->W.ctr, 0, sizeof(WaveCounters), st));
     LUX_CUDA(launch_camera_jobs(E->W, E->dopt, wave_paths, 0, st));
     for (int b = 0; b < depth; ++b) {
+        // few paths left: their remaining bounces in one launch
+        if (try_tail(b, depth))
+            LUX_CUDA(launch_paths(E->S, E->W, E->dopt, one_seg(b), depth, path_limit(kTailPerLane), st));
         LUX_CUDA(launch_trace(E->S, E->W, b, 0, nee, st, trace_grid));
         if (nee) LUX_CUDA(launch_trace(E->S, E->W, b, nee == 2 ? 2 : 1, 0, st, trace_grid));
         LUX_CUDA(launch_shade(E->S, E->W, E->dopt, b, 1, st));
@@ -386,6 +389,7 @@ int lux_engine_create(const lux_scene_desc* const* scenes, int num_scenes, const
     // occupancy queries happen here, never inside a stream capture
     for (int m = 0; m < 3; ++m) trace_grid_blocks(m, E->S.single_level != 0);
     shade_grid_blocks();
+    path_grid_blocks();
     const int full = trace_grid_blocks(0, E->S.single_level != 0);
     if (c.max_paths > 0 || c.trace_blocks > 0) {
         E->max_paths = E->paths_alloc;
@@ -618,6 +622,7 @@ int finish_pending(lux_engine* E, int* done) {
 int step_pipelined(lux_engine* E, int* done_jobs, int* idle) {
     cudaStream_t st = E->stream;
     const int nee = E->dopt.env ? 2 : (E->dopt.dl ? 1 : 0);
+    bool drain = false;  // no work waits: the waves in flight have no later one to ride along with
     if (int(E->flight.size()) < E->lanes) {
         int lane = 0;
         for (; lane < E->lanes; ++lane) {
@@ -635,6 +640,7 @@ int step_pipelined(lux_engine* E, int* done_jobs, int* idle) {
             LUX_CUDA(launch_camera_jobs(lane_view(E, lane), E->dopt, wave_paths, lane, st));
             E->flight.push_back(std::move(f));
         }
+        drain = k == 0;
     }
     if (E->flight.empty()) {
         // nothing in flight: the step enqueued last, if any, is the last to finish
@@ -657,6 +663,8 @@ int step_pipelined(lux_engine* E, int* done_jobs, int* idle) {
             ++G.n;
         }
         if (G.n == 0) break;
+        if (drain && try_tail(E->flight.back().bounce, E->flight.back().depth))
+            LUX_CUDA(launch_paths(E->S, E->W, E->dopt, G, kMaxDepth, path_limit(kTailPerLane), st));
         LUX_CUDA(launch_trace_segs(E->S, E->W, G, 0, nee, st, E->trace_blocks));
         if (nee) LUX_CUDA(launch_trace_segs(E->S, E->W, G, nee == 2 ? 2 : 1, 0, st, E->trace_blocks));
         LUX_CUDA(launch_shade_segs(E->S, E->W, E->dopt, G, st));

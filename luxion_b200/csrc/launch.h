@@ -1,6 +1,7 @@
 // launch.h -- host-callable launchers of the kernels (defined in trace.cu, shade.cu, sort.cu).
 #pragma once
 
+#include <algorithm>
 #include <cuda_runtime.h>
 #include "device_scene.h"
 
@@ -50,6 +51,21 @@ cudaError_t launch_camera(const DevScene& S, const DevWave& W, const DevOptions&
 cudaError_t launch_paths(const DevScene& S, const DevWave& W, const DevOptions& O, const Segs& G, int depth, int limit,
                          cudaStream_t st);
 int path_grid_blocks();
+// Waves of at most kWholePerLane paths per lane of the whole-path kernel's grid (284k on 148 SMs)
+// run in it from the camera on. Above, the wavefront's full warps win: 0.81 against 1.18 ms for
+// 228k paths (477k triangles) and 0.35 against 0.53 for 66k (Cornell box), but 1.65 against 1.12 ms
+// for 367k (842k triangles). A larger wave hands over before one of the bounces 1 to kTailLast once
+// at most kTailPerLane paths per lane are left (114k) and two bounces or more are to come: a frame
+// of 2.07M paths, 1M triangles, depth 12 takes 4.18 ms instead of 5.34, while handing over at
+// twice that many took 5 to 20 % longer in 700k-triangle scenes. An attempt that finds more paths
+// left costs an empty launch.
+constexpr int kWholePerLane = 5;
+constexpr int kTailPerLane = 2;
+constexpr int kTailLast = 3;
+inline int path_limit(int per_lane) { return per_lane * path_grid_blocks() * kPathBlock; }
+inline int tail_attempts(int depth) { return std::max(0, std::min(kTailLast, depth - 2)); }
+inline bool try_tail(int bounce, int depth) { return bounce >= 1 && bounce <= kTailLast && bounce + 2 <= depth; }
+
 // shade bounce `bounce` (depth = bounce + 1 after the increment of src/pathtrace.cu:264)
 cudaError_t launch_shade(const DevScene& S, const DevWave& W, const DevOptions& O, int bounce, int compact,
                          cudaStream_t st);
