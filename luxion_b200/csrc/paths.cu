@@ -45,6 +45,7 @@ struct RegPathIn {
         return mk(a.x, a.y, a.z);
     }
     LUX_DI f3 nee() const { return ns; }
+    LUX_DI void set_color(f3 c, int iter) const { W.s3[pid] = make_float4(c.x, c.y, c.z, __int_as_float(iter)); }
 };
 
 struct PathArgs {
@@ -60,8 +61,9 @@ struct PathArgs {
 // instruction caches, so the block's warps shade in step (k_shade), and one copy of the traversal
 // serves both kinds of ray. 256x256 Cornell box, depth 8 (65536 paths): 0.53 ms as a wavefront; here
 // 0.76 with warps shading at their own pace and four blocks per SM (0.59 with three, 0.55 with two),
-// in step 0.38 with four blocks, 0.35 with three (168 registers) and two, 0.39 with 256 x 2 and
-// 512 x 1. 29302 paths, 50k triangles: 0.48 as a wavefront, 0.16 here.
+// in step 0.38 with four blocks, 0.35 with three and two. With today's traversal and shading 0.32
+// (150 registers), as with 256 x 2; 0.33 with 64 x 6 and 256 x 1. 29302 paths, 50k triangles: 0.48 as
+// a wavefront, 0.15 here (0.17 with 256 x 2).
 template <bool JOBS, int NEE, bool SINGLE>
 __global__ void __launch_bounds__(kPathBlock, kPathOcc) k_paths(const __grid_constant__ PathArgs A) {
     __shared__ uint2 stack[kShStack][kPathBlock];
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(kPathBlock, kPathOcc) k_paths(const __grid_con
         bool hit = false;
 #pragma unroll 1
         for (int k = 0; k < (NEE ? 2 : 1); ++k) {
-            Tracer<NEE == 2 ? -1 : 0, SINGLE, PathKey> T{A.S, stack, hits, lut, {}, int(threadIdx.x), err, PathKey{p}, k == 1};
+            Tracer<NEE == 2 ? -1 : 0, SINGLE, kPathBlock, PathKey> T{A.S, stack, hits, lut, {}, int(threadIdx.x), err, PathKey{p}, k == 1};
             Lane L;
             bool active = has;
             if (k == 0) {
@@ -190,12 +192,12 @@ __global__ void __launch_bounds__(kPathBlock, kPathOcc) k_paths(const __grid_con
         // shading, the block's warps in step (see k_shade)
         phase<true>();
         const RegPathIn in{A.W, pid, p.o, ns, p.last_pdf};
-        const bool alive = shade_one<false, NEE, false, true>(*sp, A.O, depth, p, in, hit ? best.t : -1.0f, best.inst, best.prim,
+        RegisterPark K;
+        const bool alive = shade_one<false, NEE, false, true>(*sp, A.O, depth, p, in, K, hit ? best.t : -1.0f, best.inst, best.prim,
                                                               best.u, best.v, sh.t, NEE == 2 ? -1 : sh.inst, sh.prim, sh.u,
                                                               sh.v, has) &&
                            depth < last;
         if (has) {
-            A.W.s3[pid] = make_float4(p.color.x, p.color.y, p.color.z, __int_as_float(p.iter));
             if (alive) {
                 if (NEE) {
                     f3 ed;

@@ -97,13 +97,17 @@ __global__ void __launch_bounds__(kCameraBlock, 16) k_camera(DevScene S, DevWave
 // share each fetched line: 0.3 stall cycles, and what is left is waiting for loads (12 of 24).
 // Shade time of that scene's 16-spp step: 12.95 ms free-running; in step with 128-thread blocks
 // 13.7, 256 x 8 per SM 13.0, 512 x 4 12.2, 512 x 3 (40 registers) 11.0, 384 x 3 (56) 10.7,
-// 256 x 4 (64) 11.0, 512 x 2 (64) 11.8, 1024 x 1 11.9.
+// 256 x 4 (64) 11.0, 512 x 2 (64) 11.8, 1024 x 1 11.9. Values that wait for a later phase do so in
+// shared memory (35 KB a block) instead of being spilled: 10.7 -> 10.5, and a path whose radiance
+// does not change is not written; 384 x 4 (40 registers) 10.7, 512 x 3 10.8, 512 x 2 10.6. Prefetching
+// the next item's state to L2 or L1 took 11.2.
 // G: the (lane, bounce) segments of waves in flight this launch shades; the paths of segment k
 // are its lane's queue at its bounce, and its survivors go to the lane's next queue.
 template <bool JOBS, bool MATDBG, int NEE>
 __global__ void __launch_bounds__(kShadeBlock, kShadeOcc) k_shade(const __grid_constant__ DevScene S0, DevWave W, DevOptions O,
                                                        const __grid_constant__ Segs G) {
     __shared__ int seg_first[kMaxSegs + 1];
+    __shared__ float parked[kParked][kShadeBlock];
     if (threadIdx.x == 0) {
         int t = 0;
         seg_first[0] = 0;
@@ -158,17 +162,17 @@ __global__ void __launch_bounds__(kShadeBlock, kShadeOcc) k_shade(const __grid_c
             }
         }
         const DevScene& S = *sp;
-        alive = shade_one<MATDBG, NEE, false, !MATDBG>(S, O, depth, p, WavePathIn{W, pid}, h.x, __float_as_int(h.w), prim,
+        SharedPark K{&parked[0][threadIdx.x]};
+        alive = shade_one<MATDBG, NEE, false, !MATDBG>(S, O, depth, p, WavePathIn{W, pid}, K, h.x, __float_as_int(h.w), prim,
                                                       h.y, h.z, sh_t, si, spr, su, sv, on) &&
                 job_compact;
-        if (on) st_stream(&W.s3[pid], make_float4(p.color.x, p.color.y, p.color.z, __int_as_float(p.iter)));
         if (alive) {
             st_stream(&W.s0[pid], make_float4(p.o.x, p.o.y, p.o.z, p.last_pdf));
             st_stream(&W.s1[pid], make_float4(p.d.x, p.d.y, p.d.z, __int_as_float(p.spec ? 1 : 0)));
-            st_stream(&W.s2[pid], make_float4(p.thr.x, p.thr.y, p.thr.z, __int_as_float(p.pixel)));
+            st_stream(&W.s2[pid], make_float4(p.thr.x, p.thr.y, p.thr.z, K.get(kPkPixel)));
             if (nee) {
                 f3 ed;
-                f3 dl = light_sample<NEE>(S, O, p.iter, p.pixel, depth, ed, !nee_env<NEE>(O));
+                f3 dl = light_sample<NEE>(S, O, __float_as_int(K.get(kPkIter)), __float_as_int(K.get(kPkPixel)), depth, ed, !nee_env<NEE>(O));
                 f3 v = nee_env<NEE>(O) ? ed : dl;
                 st_stream(&W.s4[pid], make_float4(v.x, v.y, v.z, 0.0f));
             }
@@ -373,12 +377,17 @@ __global__ void k_tonemap(const float* __restrict__ image, uchar4* __restrict__ 
 // Path rows of 24 floats: origin 0-2, direction 3-5, radiance 6-8, throughput 9-11, DL point
 // 12-14, env direction 15-17, pixel 18, killed 19, specular 20, pdf 21.
 struct RowPathIn {
-    const float* f;
+    float* f;
     bool env;
     LUX_DI f3 origin() const { return mk(f[0], f[1], f[2]); }
     LUX_DI float last_pdf() const { return f[21]; }
     LUX_DI f3 color0() const { return mk(f[6], f[7], f[8]); }
     LUX_DI f3 nee() const { return env ? mk(f[15], f[16], f[17]) : mk(f[12], f[13], f[14]); }
+    LUX_DI void set_color(f3 c, int) const {
+        f[6] = c.x;
+        f[7] = c.y;
+        f[8] = c.z;
+    }
 };
 
 __global__ void k_shade_ext(DevScene S, DevOptions O, float* paths, const uint32_t* hits, int n, int iter, int depth,
@@ -403,13 +412,13 @@ __global__ void k_shade_ext(DevScene S, DevOptions O, float* paths, const uint32
             float su = __uint_as_float(h[8]), sv = __uint_as_float(h[9]);
             int si = int(h[6]), spr = int(h[7]);
             if (O.env) si = -1;
-            bool survived = shade_one<true, -1, true, false>(S, O, depth, p, RowPathIn{f, O.env != 0}, t, inst, prim,
+            RegisterPark K;
+            bool survived = shade_one<true, -1, true, false>(S, O, depth, p, RowPathIn{f, O.env != 0}, K, t, inst, prim,
                                                 __uint_as_float(h[3]), __uint_as_float(h[4]), __uint_as_float(h[5]), si,
                                                 spr, su, sv);
             alive = survived && compact;
             f[0] = p.o.x; f[1] = p.o.y; f[2] = p.o.z;
             f[3] = p.d.x; f[4] = p.d.y; f[5] = p.d.z;
-            f[6] = p.color.x; f[7] = p.color.y; f[8] = p.color.z;
             f[9] = p.thr.x; f[10] = p.thr.y; f[11] = p.thr.z;
             f[19] = survived ? 0.0f : 1.0f;
             f[20] = p.spec ? 1.0f : 0.0f;

@@ -499,16 +499,17 @@ LUX_DI f3 light_sample(const DevScene& S, const DevOptions& O, int iter, int pix
 }
 
 // A path as shade_one sees it. d, thr, spec, pixel and iter are read on entry; the other
-// fields are outputs: the new origin, radiance and pdf of a surviving path (color always).
+// fields are outputs: the new origin and pdf of a surviving path.
 struct PathState {
-    f3 o, d, thr, color;
+    f3 o, d, thr;
     float last_pdf;
     bool spec;
     int pixel, iter;
 };
 
 // The path fields shade_one reads late, loaded where they are used instead of being held in
-// registers across the shading (origin, radiance so far, pdf of the last bounce, NEE sample).
+// registers across the shading (origin, radiance so far, pdf of the last bounce, NEE sample), and
+// the radiance, written where it is known (a path without a radiance term keeps it).
 struct WavePathIn {
     const DevWave& W;
     int pid;
@@ -516,7 +517,31 @@ struct WavePathIn {
     LUX_DI float last_pdf() const { return ld_stream(&W.s0[pid]).w; }
     LUX_DI f3 color0() const { float4 a = ld_stream(&W.s3[pid]); return mk(a.x, a.y, a.z); }
     LUX_DI f3 nee() const { float4 a = ld_stream(&W.s4[pid]); return mk(a.x, a.y, a.z); }
+    LUX_DI void set_color(f3 c, int iter) const { st_stream(&W.s3[pid], make_float4(c.x, c.y, c.z, __int_as_float(iter))); }
 };
+
+// Values that wait from one phase to a later one. In the wavefront's kernel they wait in shared
+// memory (a phase's barrier makes the compiler read them back), in the others in registers.
+enum Parked {
+    kPkAlbedo = 0, kPkNormal = 3, kPkN0 = 6, kPkRough = 9, kPkMetal = 10, kPkIor = 11, kPkTrans = 12, kPkThr = 13,
+    kPkLight = 16, kPkPdf = 19, kPkCos = 20, kPkPixel = 21, kPkIter = 22, kParked = 23
+};
+struct SharedPark {
+    float* at;  // [kParked][kShadeBlock], this thread's column
+    LUX_DI void put(int i, float v) { at[i * kShadeBlock] = v; }
+    LUX_DI float get(int i) const { return at[i * kShadeBlock]; }
+};
+struct RegisterPark {
+    float v[kParked];
+    LUX_DI void put(int i, float x) { v[i] = x; }
+    LUX_DI float get(int i) const { return v[i]; }
+};
+template <class PARK> LUX_DI void put3(PARK& K, int i, f3 v) {
+    K.put(i, v.x);
+    K.put(i + 1, v.y);
+    K.put(i + 2, v.z);
+}
+template <class PARK> LUX_DI f3 get3(const PARK& K, int i) { return mk(K.get(i), K.get(i + 1), K.get(i + 2)); }
 
 // A phase boundary of the shading: the block's warps meet, so that they fetch the next phase's
 // instructions together (k_shade).
@@ -528,7 +553,7 @@ template <bool PHASED> LUX_DI void phase() {
 // sh_t: DL shadow hit t (or env occlusion); sh_* the DL shadow hit record.
 // MATDBG: the instantiation that also renders the material debug views (O.material_debug).
 // NEE: as for light_sample. At most one radiance term is added per call (emission, the NEE
-// contribution or the environment on a miss), so p.color = color0 + that term.
+// contribution or the environment on a miss).
 // SPAWN_KILLED: also sample the next direction and spawn the ray of a path that an emitter
 // hit kills, as the reference does (its result is then unused; the parity entry reports it).
 // The NEE terms draw no random numbers, so sampling the direction after them leaves the
@@ -540,175 +565,192 @@ template <bool PHASED> LUX_DI void phase() {
 // environment step with the hits that sample it, and the two BSDF evaluations of a hit share
 // theirs. on: false for a lane that only takes part in the phases (PHASED needs every thread of
 // the block; the results of such a lane are not read).
-template <bool MATDBG, int NEE, bool SPAWN_KILLED, bool PHASED, class In>
-LUX_DI bool shade_one(const DevScene& S, const DevOptions& O, int depth, PathState& p, const In& in, float t, int inst,
-                      int prim, float bu, float bv, float sh_t, int sh_inst, int sh_prim, float sh_u, float sh_v,
+template <bool MATDBG, int NEE, bool SPAWN_KILLED, bool PHASED, class In, class PARK>
+LUX_DI bool shade_one(const DevScene& S, const DevOptions& O, int depth, PathState& p, const In& in, PARK& K, float t,
+                      int inst, int prim, float bu, float bv, float sh_t, int sh_inst, int sh_prim, float sh_u, float sh_v,
                       bool on = true) {
     Rng rng = Rng::seeded(p.iter, p.pixel, depth);
-    f3 add = mk(0.0f, 0.0f, 0.0f);
-    bool added = false;
+    K.put(kPkPixel, __int_as_float(p.pixel));
+    K.put(kPkIter, __int_as_float(p.iter));
+    put3(K, kPkThr, p.thr);
     const bool has_exr = S.has_env != 0;
     const bool hit = on && inst >= 0 && t > 0.0f;
     const bool miss = on && !hit;
-    const f3 wo = -p.d;
-    // ---- surface
-    f3 mc, normal, n0, emission;
-    float rough = 0.0f, metal = 0.0f, ior = 1.0f, trans = 0.0f;
     bool emissive = false;
-    mc = normal = n0 = emission = mk(0.0f, 0.0f, 0.0f);
+    // ---- surface
     if (hit) {
         const Isect is = ch_radiance(S, t, inst, prim, bu, bv);
         const DevMaterial& m = S.mats[is.material];
-        mc = get_albedo(m, is.u, is.v);
-        normal = get_normal(S, m, is);
-        n0 = is.normal;
+        const f3 mc = get_albedo(m, is.u, is.v);
+        const f3 normal = get_normal(S, m, is);
+        float rough, metal;
         get_mr(m, is.u, is.v, rough, metal);
         if (MATDBG && O.material_debug) {
             // the debug view replaces the colour and ends the path (shade_path.cu:154-164)
-            p.color = material_debug_color(O.material_debug, mc, normal, normal_map_texel(m, is.u, is.v), rough, metal,
-                                           get_alpha(m, is.u, is.v));
+            in.set_color(material_debug_color(O.material_debug, mc, normal, normal_map_texel(m, is.u, is.v), rough, metal,
+                                              get_alpha(m, is.u, is.v)),
+                         p.iter);
             return false;
         }
-        emission = get_emission(m, is.u, is.v);
+        const f3 emission = get_emission(m, is.u, is.v);
         emissive = length(emission) > kEPS_UTIL;
-        ior = gmax(m.ior, 1.0001f);
-        trans = m.transmission;
+        put3(K, kPkAlbedo, mc);
+        put3(K, kPkNormal, normal);
+        put3(K, kPkN0, is.normal);
+        K.put(kPkRough, rough);
+        K.put(kPkMetal, metal);
+        K.put(kPkIor, gmax(m.ior, 1.0001f));
+        K.put(kPkTrans, m.transmission);
+        put3(K, kPkLight, emission);
     }
     phase<PHASED>();
-    const bool is_spec = rough < kSPEC_ROUGH;
-    const f3 nf = dot(wo, normal) < 0.0f ? -normal : normal;
+    // ---- light: the sample of a hit that sees it (lit), emission, environment
     // MIS applies to the light a BSDF sample found (not for camera rays and specular bounces)
     const bool mis = depth > 1 && !p.spec;
-    const bool kill_light = hit && emissive;
-    // ---- light: pl, le, cs are the light sample's pdf, radiance and cosine, wl its direction,
-    // for hits whose sample is visible (lit)
     bool lit = false;
-    f3 wl = mk(0.0f, 0.0f, 0.0f), le = wl;
-    float pl = 0.0f, cs = 0.0f;
-    float w = 1.0f;  // MIS weight of emission or the environment found by the BSDF
-    if (nee_env<NEE>(O)) {
-        if (hit && !emissive && sh_t < 0.0f && !is_spec && has_exr) {
-            wl = in.nee();
-            cs = dot(nf, wl);
-            lit = cs > 0.0f;  // a sample below the horizon contributes nothing
+    f3 wl = mk(0.0f, 0.0f, 0.0f);
+    {
+        float pl = 0.0f;
+        float w = 1.0f;  // MIS weight of emission or the environment found by the BSDF
+        if (nee_env<NEE>(O)) {
+            if (hit && !emissive && sh_t < 0.0f && !(K.get(kPkRough) < kSPEC_ROUGH) && has_exr) {
+                const f3 normal = get3(K, kPkNormal);
+                wl = in.nee();
+                const float cs = dot(dot(-p.d, normal) < 0.0f ? -normal : normal, wl);
+                lit = cs > 0.0f;  // a sample below the horizon contributes nothing
+                K.put(kPkCos, cs);
+            }
         }
-    }
-    if (has_exr && (miss || (hit && nee_env<NEE>(O)))) {
-        const f3 dm = hit ? p.d : normalize(p.d);
-        f3 d = lit ? wl : dm;
-        bool pdf = lit || (nee_env<NEE>(O) && mis && (!hit || emissive));
-        bool look = !hit && !pdf;
-        // a hit's sample takes the pdf of its direction and the radiance of the normalised one;
-        // a miss takes both of one direction
-        if (pdf || look) {
+        if (has_exr && (miss || (hit && nee_env<NEE>(O)))) {
+            f3 d = lit ? wl : hit ? p.d : normalize(p.d);
+            bool pdf = lit || (nee_env<NEE>(O) && mis && (miss || emissive));
+            bool look = miss && !pdf;
+            // a hit's sample takes the pdf of its direction and the radiance of the normalised one;
+            // a miss takes both of one direction
+            if (pdf || look) {
 #pragma unroll 1
-            while (true) {
-                float phi, theta;
-                env_angles(d, phi, theta);
-                if (pdf) {
-                    pl = envmap_pdf(S, phi, theta);
-                    pdf = false;
-                    if (lit && pl > 1e-8f) {
-                        d = normalize(wl);
-                        look = true;
-                        continue;
+                while (true) {
+                    float phi, theta;
+                    env_angles(d, phi, theta);
+                    if (pdf) {
+                        pl = envmap_pdf(S, phi, theta);
+                        pdf = false;
+                        if (lit && pl > 1e-8f) {
+                            d = normalize(wl);
+                            look = true;
+                            continue;
+                        }
+                        look = miss;
                     }
-                    look = !hit;
+                    if (look) put3(K, kPkLight, env_lookup(S, phi, theta, O.env_intensity));
+                    break;
                 }
-                if (look) le = env_lookup(S, phi, theta, O.env_intensity);
-                break;
+            }
+            if (lit) {
+                lit = pl > 1e-8f;
+                K.put(kPkPdf, pl);
+            } else if (mis && nee_env<NEE>(O) && (miss || emissive)) {
+                const float pb = in.last_pdf();
+                w = (pb * pb) / (pb * pb + pl * pl);
             }
         }
-        if (lit) lit = pl > 1e-8f;
-        else if (mis && (nee_env<NEE>(O)) && (!hit || emissive)) {
-            const float pb = in.last_pdf();
-            w = (pb * pb) / (pb * pb + pl * pl);
-        }
-    }
-    if (nee_dl<NEE>(O) && !nee_env<NEE>(O) && hit) {
-        if (emissive) {
-            if (mis) {
-                float pb = in.last_pdf();
-                float dsq = t * t;
-                float cl = dot(n0, wo);
-                if (cl > 0.0001f) {
+        if (nee_dl<NEE>(O) && !nee_env<NEE>(O) && hit) {
+            if (emissive) {
+                if (mis) {
+                    float pb = in.last_pdf();
+                    float dsq = t * t;
+                    float cl = dot(get3(K, kPkN0), -p.d);
+                    if (cl > 0.0001f) {
+                        float pa = 1.0f / S.total_area;
+                        float ps = pa * (dsq / cl);
+                        w = (pb * pb) / (pb * pb + ps * ps);
+                    } else {
+                        w = 0.0f;
+                    }
+                }
+            } else if (sh_inst >= 0 && sh_t > 0.0f && !(K.get(kPkRough) < kSPEC_ROUGH)) {
+                Isect dli = ch_direct_light(S, sh_t, sh_inst, sh_prim, sh_u, sh_v);
+                f3 sp = t * p.d + in.origin();
+                f3 lv = in.nee() - sp;
+                float dsq = dot(lv, lv);
+                float dist = sqrtf(dsq);
+                wl = lv / dist;
+                const f3 normal = get3(K, kPkNormal);
+                const float cs = dot(dot(-p.d, normal) < 0.0f ? -normal : normal, wl);
+                float cl = dot(dli.normal, -wl);
+                if (cs > 0.0f && cl > 0.0f) {
                     float pa = 1.0f / S.total_area;
-                    float ps = pa * (dsq / cl);
-                    w = (pb * pb) / (pb * pb + ps * ps);
-                } else {
-                    w = 0.0f;
+                    const DevMaterial& lm = S.mats[dli.material];
+                    K.put(kPkCos, cs);
+                    K.put(kPkPdf, pa * (dsq / cl));
+                    put3(K, kPkLight, get_emission(lm, dli.u, dli.v));
+                    lit = true;
                 }
             }
-        } else if (sh_inst >= 0 && sh_t > 0.0f && !is_spec) {
-            Isect dli = ch_direct_light(S, sh_t, sh_inst, sh_prim, sh_u, sh_v);
-            f3 sp = t * p.d + in.origin();
-            f3 lv = in.nee() - sp;
-            float dsq = dot(lv, lv);
-            float dist = sqrtf(dsq);
-            wl = lv / dist;
-            cs = dot(nf, wl);
-            float cl = dot(dli.normal, -wl);
-            if (cs > 0.0f && cl > 0.0f) {
-                float pa = 1.0f / S.total_area;
-                pl = pa * (dsq / cl);
-                const DevMaterial& lm = S.mats[dli.material];
-                le = get_emission(lm, dli.u, dli.v);
-                lit = true;
-            }
+        }
+        // radiance a path without a BSDF step ends with (at most one term is added per call)
+        if (miss ? has_exr : emissive) {
+            const f3 thr = get3(K, kPkThr), le = get3(K, kPkLight);
+            const f3 add = miss ? thr * le * w : (nee_env<NEE>(O) || nee_dl<NEE>(O)) ? thr * (w * le) : thr * le;
+            in.set_color(in.color0() + add, __float_as_int(K.get(kPkIter)));
         }
     }
     phase<PHASED>();
-    bool kill = kill_light;
-    bool done = !hit;  // no BSDF step: a miss, or an emitter hit whose ray is not spawned
-    if (miss) {
-        if (has_exr) {
-            add = p.thr * le * w;
-            added = true;
-        }
-    } else if (hit && emissive) {
-        add = (nee_env<NEE>(O) || nee_dl<NEE>(O)) ? p.thr * (w * emission) : p.thr * emission;
-        added = true;
-        done = !SPAWN_KILLED;
-    }
+    bool kill = emissive;
+    const bool done = !hit || (emissive && !SPAWN_KILLED);  // no BSDF step
     // ---- BSDF: k = 0 for the light's direction, k = 1 for the sampled one
-    Lobes L;
-    L.pR = L.pD = L.pS = 0.0f;
-    if (!done) L = lobes_of(wo, normal, metal, mc, ior, trans);
     f3 sd = mk(0.0f, 0.0f, 0.0f);
-#pragma unroll 1
-    for (int k = NEE == 0 ? 1 : 0; k < 2; ++k) {
-        if (k == 1) {
-            if (!done) sd = sample_ct(wo, normal, rough, rng, ior, L);
-            phase<PHASED>();
+    {
+        f3 normal = mk(0.0f, 0.0f, 1.0f), mc = normal;
+        float rough = 1.0f, metal = 0.0f, ior = 1.5f, trans = 0.0f;
+        Lobes L;
+        L.pR = L.pD = L.pS = 0.0f;
+        const f3 wo = -p.d;
+        if (!done) {
+            mc = get3(K, kPkAlbedo);
+            normal = get3(K, kPkNormal);
+            rough = K.get(kPkRough);
+            metal = K.get(kPkMetal);
+            ior = K.get(kPkIor);
+            trans = K.get(kPkTrans);
+            L = lobes_of(wo, normal, metal, mc, ior, trans);
         }
-        if (!(done || (k == 0 ? !lit : kill))) {
-            const f3 wi = k == 0 ? wl : sd;
-            const bool refr = (dot(wi, normal) * dot(wo, normal)) < 0.0f;
-            const float pdf = PDF(wo, wi, normal, rough, ior, L);
-            const f3 f = (k == 1 && refr) ? BTDF(wo, normal, wi, mc, rough, metal, ior, trans)
-                                          : BRDF(wo, normal, wi, mc, rough, metal, ior, trans);
-            if (k == 0) {
-                const float wt = (pl * pl) / (pl * pl + pdf * pdf);
-                f3 contrib = (le * f * cs) / pl;
-                add = p.thr * contrib * wt;
-                added = true;
-            } else {
-                p.thr = p.thr * ((f * fabsf(dot(wi, normal))) / pdf);
-                p.last_pdf = pdf;
-                p.spec = is_spec || refr;
-                if (depth >= kRR_MIN_DEPTH) {
-                    float mx = gmax(p.thr.x, gmax(p.thr.y, p.thr.z));
-                    float surv = gclamp(mx, 0.0f, 1.0f);
-                    if (rng.u01() >= surv) kill = true;
-                    else p.thr = p.thr / surv;
+#pragma unroll 1
+        for (int k = NEE == 0 ? 1 : 0; k < 2; ++k) {
+            if (k == 1) {
+                if (!done) sd = sample_ct(wo, normal, rough, rng, ior, L);
+                phase<PHASED>();
+            }
+            if (!(done || (k == 0 ? !lit : kill))) {
+                const f3 wi = k == 0 ? wl : sd;
+                const bool refr = (dot(wi, normal) * dot(wo, normal)) < 0.0f;
+                const float pdf = PDF(wo, wi, normal, rough, ior, L);
+                const f3 f = (k == 1 && refr) ? BTDF(wo, normal, wi, mc, rough, metal, ior, trans)
+                                              : BRDF(wo, normal, wi, mc, rough, metal, ior, trans);
+                const f3 thr = get3(K, kPkThr);
+                if (k == 0) {
+                    const float pl = K.get(kPkPdf), cs = K.get(kPkCos);
+                    const float wt = (pl * pl) / (pl * pl + pdf * pdf);
+                    f3 contrib = (get3(K, kPkLight) * f * cs) / pl;
+                    in.set_color(in.color0() + thr * contrib * wt, __float_as_int(K.get(kPkIter)));
+                } else {
+                    p.thr = thr * ((f * fabsf(dot(wi, normal))) / pdf);
+                    p.last_pdf = pdf;
+                    p.spec = rough < kSPEC_ROUGH || refr;
+                    if (depth >= kRR_MIN_DEPTH) {
+                        float mx = gmax(p.thr.x, gmax(p.thr.y, p.thr.z));
+                        float surv = gclamp(mx, 0.0f, 1.0f);
+                        if (rng.u01() >= surv) kill = true;
+                        else p.thr = p.thr / surv;
+                    }
                 }
             }
+            phase<PHASED>();
         }
-        phase<PHASED>();
     }
-    if (on) p.color = added ? in.color0() + add : in.color0();
     if (done) return false;
     // ray spawn (shade_path.cu:333-353), run for paths killed above as well
+    const f3 n0 = get3(K, kPkN0);
     f3 hp = in.origin() + (t - .0001f) * normalize(p.d);
     float sl2 = dot(sd, sd);
     if (!(sl2 > 1e-12f) || !isfinite(sl2)) return false;

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kTraceBlock, SINGLE ? 7 : 6) k_trace(const __g
         }
     }
     __syncthreads();
-    Tracer<MODE, SINGLE, RayKey<EXT>> T{A.S, stack, hits, lut, {}, int(threadIdx.x), EXT ? A.ext_err : &(A.W.ctr + A.G.lane[0])->error,
+    Tracer<MODE, SINGLE, kTraceBlock, RayKey<EXT>> T{A.S, stack, hits, lut, {}, int(threadIdx.x), EXT ? A.ext_err : &(A.W.ctr + A.G.lane[0])->error,
                                         RayKey<EXT>{A}, MODE == 2};
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;

@@ -273,10 +273,10 @@ struct Lane {
 // MODE: 0 radiance, 1 DL shadow, 2 env occlusion (any hit), 3 BVH heatmap; -1: `any` says at run
 // time whether any hit ends the ray (one copy of the code for both kinds of ray).
 // KEY: gives the pixel and iteration that key a ray's alpha-blend hash, from Lane::key.
-template <int MODE, bool SINGLE, class KEY>
+template <int MODE, bool SINGLE, int BLOCK, class KEY>
 struct Tracer {
     const DevScene& S;
-    uint2 (*sh)[kTraceBlock];  // shared stack [kShStack][block]
+    uint2 (*sh)[BLOCK];  // shared stack [kShStack][block]
     float4* hits;              // shared, per thread: the closest hit's u, v, instance, prim (int bits)
     const unsigned char* lut;  // shared, fill_key_table
     uint2 loc[kLocStack];
