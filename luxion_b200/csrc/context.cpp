@@ -34,6 +34,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <tuple>
 #include <vector>
@@ -1205,8 +1206,8 @@ struct PinnedBlock {
 // memory copies overlap one another and the DMA. The driver's own pageable copy stages on one
 // thread: with it, and a cudaMalloc and cudaFree per buffer, 300,001 rays took 3.3 ms a call, now 1.1
 // to 1.4.
-// All copies are on stream st; the call returns with those to the host complete and those to the
-// device enqueued and read from the caller's memory.
+// All copies are on stream st; the call returns with those to the host complete (or, without
+// page-locked memory, enqueued) and those to the device enqueued and read from the caller's memory.
 constexpr size_t kCopyChunk = size_t(512) << 10;
 constexpr int kCopyThreads = 3;
 // Copies smaller than this go through the driver: below it the threads cost more than they save
@@ -1219,7 +1220,12 @@ int staged_copy(int device, cudaStream_t st, void* dev, void* host, size_t bytes
     const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
     const int nt = std::max(1, std::min({kCopyThreads, int(hw / 2), chunks / 2}));
     PinnedBlock stage(size_t(nt) * 2 * kCopyChunk);
-    if (!stage.p) return fail(LUX_ERR_OOM, "page-locked host allocation failed");
+    if (!stage.p) {  // no page-locked memory to be had: the driver's own staging
+        cudaGetLastError();
+        LUX_CUDA(cudaMemcpyAsync(to_device ? dev : host, to_device ? host : dev, bytes,
+                                 to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, st));
+        return LUX_OK;
+    }
     std::atomic<int> failed{0};
     auto work = [&](int t) {
         char* slot[2];
@@ -1263,10 +1269,15 @@ int staged_copy(int device, cudaStream_t st, void* dev, void* host, size_t bytes
             }
         if (e != cudaSuccess) failed = int(e);
     };
-    std::vector<std::thread> th;
-    for (int t = 1; t < nt; ++t) th.emplace_back(work, t);
+    std::thread th[kCopyThreads];
+    int started = 1;
+    try {
+        for (; started < nt; ++started) th[started] = std::thread(work, started);
+    } catch (const std::system_error&) {  // no thread to be had: its chunks are moved here
+    }
     work(0);
-    for (auto& t : th) t.join();
+    for (int t = started; t < nt; ++t) work(t);
+    for (int t = 1; t < started; ++t) th[t].join();
     if (failed) return fail(LUX_ERR_CUDA, std::string("staged copy: ") + cudaGetErrorString(cudaError_t(failed.load())));
     return LUX_OK;
 }
