@@ -12,11 +12,11 @@
 //
 // Compiled with --fmad=false, as shade.cu is.
 
+#include "path_segs.h"
 #include "trace_core.cuh"
 #include "shade_core.cuh"
 
 #include <algorithm>
-#include <array>
 #include <map>
 #include <mutex>
 
@@ -70,36 +70,24 @@ __global__ void __launch_bounds__(kPathBlock, kPathOcc) k_paths(const __grid_con
     __shared__ float4 hits[kPathBlock];
     __shared__ unsigned char lut[2048];
     fill_key_table(lut);  // read after the barrier below
-    __shared__ int seg_first[kMaxSegs + 1];
+    __shared__ PathSegs segs;
     // this block's share of the counters: survivors entering each bounce and shadow rays
     __shared__ int n_path[kMaxSegs][kMaxDepth + 1], n_shadow[kMaxSegs][kMaxDepth];
-    if (threadIdx.x == 0) {
-        int t = 0;
-        seg_first[0] = 0;
-        for (int k = 0; k < kMaxSegs; ++k) {
-            if (k < A.G.n) {
-                const WaveCounters* c = A.W.ctr + A.G.lane[k];
-                const int f = *(volatile const int*)&c->finished;  // this launch sets bounce + 1
-                if (f == 0 || f == A.G.bounce[k] + 1) t += *(volatile const int*)&c->count[A.G.bounce[k]];
-            }
-            seg_first[k + 1] = t;
-        }
-    }
+    if (threadIdx.x == 0) segs = path_segments(A.W.ctr, A.G);
     for (int i = threadIdx.x; i < kMaxSegs * (kMaxDepth + 1); i += kPathBlock) (&n_path[0][0])[i] = 0;
     for (int i = threadIdx.x; i < kMaxSegs * kMaxDepth; i += kPathBlock) (&n_shadow[0][0])[i] = 0;
     __syncthreads();
-    const int total = seg_first[kMaxSegs];
+    const int total = segs.first[kMaxSegs];
     if (total == 0 || total > A.limit) return;
-    // the wavefront launches that follow find these lanes finished
-    if (blockIdx.x == 0 && int(threadIdx.x) < A.G.n) (A.W.ctr + A.G.lane[threadIdx.x])->finished = A.G.bounce[threadIdx.x] + 1;
+    if (blockIdx.x == 0 && int(threadIdx.x) < A.G.n) mark_segment(A.W.ctr, A.G, threadIdx.x);
 
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     // Fewer paths than lanes: every warp gets the same share, so that a path waits for few others.
     const int warps = int(gridDim.x) * (kPathBlock / 32);
     const int cap = min(32, (total + warps - 1) / warps);
-    int* cursor = &(A.W.ctr + A.G.lane[0])->fetch_p;
-    int* err = &(A.W.ctr + A.G.lane[0])->error;
+    int* cursor = &(A.W.ctr + segs.lane)->fetch_p;
+    int* err = &(A.W.ctr + segs.lane)->error;
     bool first = true, exhausted = false;  // warp-uniform
     bool has = false;
     PathState p{};
@@ -124,9 +112,9 @@ __global__ void __launch_bounds__(kPathBlock, kPathOcc) k_paths(const __grid_con
             const int r = base + __popc(need & ((1u << lane) - 1u));
             if (!has && lane < cap && r < total) {
                 seg = 0;
-                while (seg + 1 < A.G.n && r >= seg_first[seg + 1]) ++seg;
+                while (seg + 1 < A.G.n && r >= segs.first[seg + 1]) ++seg;
                 const int b = A.G.bounce[seg];
-                pid = ld_stream(&A.W.queue[b & 1][A.G.lane[seg] * A.W.lane_stride + (r - seg_first[seg])]);
+                pid = ld_stream(&A.W.queue[b & 1][A.G.lane[seg] * A.W.lane_stride + (r - segs.first[seg])]);
                 depth = b + 1;
                 last = A.depth;
                 if (JOBS) {
