@@ -18,19 +18,27 @@ namespace lux {
 
 struct PathSegs {
     int first[kMaxSegs + 1];  // paths of segment k: [first[k], first[k + 1]) of the launch's list
-    int lane;                 // the lane whose cursor and error word serve the launch
+    int lane;                 // the lane whose cursor and error word serve the launch: the first taken
 };
 
+// The cursor is that of a lane the launch takes: a lane is taken once in its wave's life, so its
+// cursor is still at the zero the wave started with. Any other lane's may have served before, and
+// the paths it has counted off would be skipped.
 LUX_SEG_FN PathSegs path_segments(const WaveCounters* ctr, const Segs& G) {
     PathSegs s;
     s.lane = G.lane[0];
     s.first[0] = 0;
+    bool any = false;
     for (int k = 0; k < kMaxSegs; ++k) {
         int t = 0;
         if (k < G.n) {
             const WaveCounters* c = ctr + G.lane[k];
             const int f = *(volatile const int*)&c->finished;  // this launch sets bounce + 1
-            if (f == 0 || f == G.bounce[k] + 1) t = *(volatile const int*)&c->count[G.bounce[k]];
+            if (f == 0 || f == G.bounce[k] + 1) {
+                t = *(volatile const int*)&c->count[G.bounce[k]];
+                if (!any) s.lane = G.lane[k];
+                any = true;
+            }
         }
         s.first[k + 1] = s.first[k] + t;
     }

@@ -24,3 +24,7 @@ def cases(tmp_path_factory):
 
 def test_blocks_agree_whenever_they_start(cases):
     assert [c for c in cases if c[3] != "agree"] == []
+
+
+def test_every_path_not_yet_finished_is_taken_once(cases):
+    assert [c for c in cases if c[4] != "cover"] == []
