@@ -312,8 +312,8 @@ int lux_wave_counts(lux_ctx* ctx, int* paths, int* shadow, int max_bounces);
  * mode 2 only word 0 is meaningful (1.0 occluded, -1.0 free). Host buffers. */
 int lux_trace_rays(lux_ctx* ctx, const float* rays, int n, int mode, int iter, uint32_t* hits);
 
-/* lux_trace_rays_static: lux_trace_rays for callers that must not allocate device memory on
- * the call. No counterpart in the reference. Same arguments, results and errors as
+/* lux_trace_rays_static: lux_trace_rays for callers that must not allocate device or page-locked
+ * memory on the call. No counterpart in the reference. Same arguments, results and errors as
  * lux_trace_rays, for n <= LUX_TRACE_STATIC_MAX_RAYS; a larger n is rejected with
  * LUX_ERR_INVALID before any device work.
  * Who needs it: a host that has given the device's free memory to its own pool or to other
@@ -324,9 +324,9 @@ int lux_trace_rays(lux_ctx* ctx, const float* rays, int n, int mode, int iter, u
  * looked up (cudaGetSymbolAddress) on every call; the first call on a device may load the
  * library's device code there, so make that first call before any stream capture begins on
  * that device.
- * Must start at zero: the traversal's work cursor in that array, which the call clears on the
- * context's stream before its launch, and its error word, which is in page-locked host memory of
- * the call. Nothing else carries over from one call to the next.
+ * Must start at zero: the traversal's work cursor in that array and its error word, in page-locked
+ * host memory that the context holds from its creation (in that array too where none was to be
+ * had); the call clears both before its launch. Nothing else carries over from one call to the next.
  * Calls that overlap on one device (two threads, or two contexts on the same device) share
  * the array and race: the library does not lock it, so serialise such calls. */
 #define LUX_TRACE_STATIC_MAX_RAYS 65536

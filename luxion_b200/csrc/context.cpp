@@ -129,6 +129,7 @@ struct lux_ctx {
     int* h_wave_iter = nullptr;          // pinned, two ints per wave of the current call
     WaveCounters* h_ctr = nullptr;       // pinned, one per wave of the current call
     int h_cap = 0;
+    int* trace_err = nullptr;            // pinned, error word of lux_trace_rays_static (null: none was to be had)
     // lanes of the wave arrays (waves in flight at once) and the lane of the last wave rendered
     int lanes = 1;
     int last_lane = 0;
@@ -1282,20 +1283,22 @@ int staged_copy(int device, cudaStream_t st, void* dev, void* host, size_t bytes
     return LUX_OK;
 }
 
-// Traces n caller rays through the device buffers of sc and waits for the hits.
-int trace_direct(lux_ctx* C, const float* rays, int n, int mode, int iter, uint32_t* hits, const TraceScratch& sc) {
+// Traces n caller rays through the device buffers of sc and waits for the hits. word: the error
+// word, page-locked; without one (null) the device word beside the cursor serves and is copied down.
+int trace_direct(lux_ctx* C, const float* rays, int n, int mode, int iter, uint32_t* hits, const TraceScratch& sc,
+                 int* word) {
     const size_t in = size_t(n) * 8 * sizeof(float), out = size_t(n) * 5 * sizeof(uint32_t);
-    PinnedBlock err(sizeof(int));
-    if (!err.p) return fail(LUX_ERR_OOM, "page-locked host allocation failed");
-    volatile int* failed = static_cast<int*>(err.p);
-    *failed = 0;
+    volatile int* failed = word;
+    int copied = 0;
+    if (failed) *failed = 0;
     if (in >= kCopyStaged) {
         if (int rc = staged_copy(C->device, C->stream, sc.rays, const_cast<float*>(rays), in, true)) return rc;
     } else {
         LUX_CUDA(cudaMemcpyAsync(sc.rays, rays, in, cudaMemcpyHostToDevice, C->stream));
     }
-    LUX_CUDA(cudaMemsetAsync(sc.cursor, 0, sizeof(int), C->stream));
-    cudaError_t e = launch_trace_ext(C->S, C->W, sc.rays, sc.hits, n, mode, iter, sc.cursor, static_cast<int*>(err.p), C->stream);
+    int* dev_word = sc.cursor + 1;
+    LUX_CUDA(cudaMemsetAsync(sc.cursor, 0, 2 * sizeof(int), C->stream));
+    cudaError_t e = launch_trace_ext(C->S, C->W, sc.rays, sc.hits, n, mode, iter, sc.cursor, word ? word : dev_word, C->stream);
     int rc = e == cudaSuccess ? LUX_OK : fail(LUX_ERR_CUDA, cudaGetErrorString(e));
     if (!rc) {
         if (out >= kCopyStaged) {
@@ -1305,11 +1308,15 @@ int trace_direct(lux_ctx* C, const float* rays, int n, int mode, int iter, uint3
             if (e != cudaSuccess) rc = fail(LUX_ERR_CUDA, cudaGetErrorString(e));
         }
     }
+    if (!rc && !word) {
+        e = cudaMemcpyAsync(&copied, dev_word, sizeof(int), cudaMemcpyDeviceToHost, C->stream);
+        if (e != cudaSuccess) rc = fail(LUX_ERR_CUDA, cudaGetErrorString(e));
+    }
     // the kernel may write the error word until it has ended, so the wait comes first either way
     e = cudaStreamSynchronize(C->stream);
     if (rc) return rc;
     if (e != cudaSuccess) return fail(LUX_ERR_CUDA, cudaGetErrorString(e));
-    if (*failed) return fail(LUX_ERR_UNSUPPORTED, "traversal stack overflow");
+    if (failed ? *failed : copied) return fail(LUX_ERR_UNSUPPORTED, "traversal stack overflow");
     return LUX_OK;
 }
 
@@ -1371,7 +1378,21 @@ size_t pinned_class(size_t bytes) {
 }
 }  // namespace
 
+namespace {
+thread_local int t_pinned_fails = 0;  // calls of pinned_get on this thread that are still to fail
+}
+
+int lux::lux_test_fail_pinned(int calls) {
+    const int left = t_pinned_fails;
+    t_pinned_fails = calls;
+    return left;
+}
+
 void* lux::pinned_get(size_t bytes) {
+    if (t_pinned_fails > 0) {
+        --t_pinned_fails;
+        return nullptr;
+    }
     const size_t c = pinned_class(bytes);
     {
         std::lock_guard<std::mutex> lk(g_pinned_mu);
@@ -1576,6 +1597,8 @@ int ctx_finish(lux_ctx* C) {
     for (int m = 0; m < 4; ++m) trace_grid_blocks(m, C->S.single_level != 0);
     shade_grid_blocks();
     path_grid_blocks();
+    C->trace_err = static_cast<int*>(pinned_get(sizeof(int)));
+    if (!C->trace_err) cudaGetLastError();  // lux_trace_rays_static does without
     if (cudaStreamSynchronize(C->stream) != cudaSuccess) return fail(LUX_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
     if (cudaGetLastError() != cudaSuccess) return fail(LUX_ERR_CUDA, "context set-up failed");
     return LUX_OK;
@@ -1769,6 +1792,7 @@ int lux_free(lux_ctx* C) {
     wave_block_put(C->device, C->wave_block, C->wave_block_bytes, C->stream);
     pinned_put(C->h_wave_iter, sizeof(int) * 2 * size_t(C->h_cap));
     pinned_put(C->h_ctr, sizeof(WaveCounters) * size_t(C->h_cap));
+    pinned_put(C->trace_err, sizeof(int));
     for (auto e : C->kev) cudaEventDestroy(e);
     if (C->ev[0]) cudaEventDestroy(C->ev[0]);
     if (C->ev[1]) cudaEventDestroy(C->ev[1]);
@@ -1822,7 +1846,9 @@ int lux_trace_rays(lux_ctx* C, const float* rays, int n, int mode, int iter, uin
     char* base = static_cast<char*>(block.p);
     TraceScratch sc{reinterpret_cast<int*>(base), reinterpret_cast<float*>(base + 256),
                     reinterpret_cast<uint32_t*>(base + 256 + ray_bytes)};
-    return trace_direct(C, rays, n, mode, iter, hits, sc);
+    PinnedBlock err(sizeof(int));
+    if (!err.p) cudaGetLastError();
+    return trace_direct(C, rays, n, mode, iter, hits, sc, static_cast<int*>(err.p));
 }
 
 int lux_trace_rays_static(lux_ctx* C, const float* rays, int n, int mode, int iter, uint32_t* hits) {
@@ -1837,7 +1863,7 @@ int lux_trace_rays_static(lux_ctx* C, const float* rays, int n, int mode, int it
     LUX_CUDA(cudaSetDevice(C->device));
     TraceScratch sc;
     LUX_CUDA(trace_static_scratch(C->device, sc));
-    return trace_direct(C, rays, n, mode, iter, hits, sc);
+    return trace_direct(C, rays, n, mode, iter, hits, sc, C->trace_err);
 }
 
 int lux_morton_keys(lux_ctx* C, const float* rays, int n, uint32_t* keys) {

@@ -47,6 +47,9 @@ void note_device_alloc();
 // still queued on any stream.
 void* pinned_get(size_t bytes);
 void pinned_put(void* p, size_t bytes);
+// For the tests: the calling thread's next `calls` calls of pinned_get find no page-locked memory
+// (free list included). Returns how many of an earlier setting have not been made.
+extern "C" int lux_test_fail_pinned(int calls);
 
 template <class T>
 int dalloc(T** p, size_t n) {

@@ -27,14 +27,16 @@ cudaError_t launch_trace(const DevScene& S, const DevWave& W, int bounce, int mo
 cudaError_t launch_trace_segs(const DevScene& S, const DevWave& W, const Segs& G, int mode, int nee, cudaStream_t st,
                               int grid = 0);
 // trace caller rays (device buffers), n * 8 floats -> n * 5 words; fetch is a zeroed int, err a
-// zeroed int the host can read (page-locked): nonzero after a traversal stack overflow
+// zeroed int (page-locked, so that the host can read it, or on the device): nonzero after a
+// traversal stack overflow
 cudaError_t launch_trace_ext(const DevScene& S, const DevWave& W, const float* rays, uint32_t* hits, int n, int mode,
                              int iter, int* fetch, int* err, cudaStream_t st);
 
 // the fixed scratch of lux_trace_rays_static on `device` (trace_static.cu), which must be the
-// current device on the first call for it: cursor, then LUX_TRACE_STATIC_MAX_RAYS rays and hits
+// current device on the first call for it: cursor and error word, then LUX_TRACE_STATIC_MAX_RAYS rays
+// and hits
 struct TraceScratch {
-    int* cursor;
+    int* cursor;  // cursor[1]: the error word where there is no page-locked one
     float* rays;
     uint32_t* hits;
 };

@@ -45,7 +45,7 @@ struct TraceArgs {
     int ext_n;
     int ext_iter;
     int* ext_fetch;
-    int* ext_err;           // and its error word, which the host can read (page-locked)
+    int* ext_err;           // and its error word, page-locked or on the device
 };
 
 

@@ -16,7 +16,7 @@
 namespace lux {
 namespace {
 
-constexpr size_t kHeaderBytes = 256;  // work cursor (int) at offset 0, rest unused
+constexpr size_t kHeaderBytes = 256;  // work cursor (int) at offset 0, error word (int) at 4, rest unused
 constexpr size_t kRayBytes = size_t(LUX_TRACE_STATIC_MAX_RAYS) * 8 * sizeof(float);
 constexpr size_t kHitBytes = size_t(LUX_TRACE_STATIC_MAX_RAYS) * 5 * sizeof(uint32_t);
 static_assert(kRayBytes % 256 == 0, "hit region starts 256-byte aligned");
