@@ -1216,6 +1216,19 @@ constexpr int kCopyThreads = 3;
 // 0.96; 1,000,000: 6.8 and 3.3).
 constexpr size_t kCopyStaged = size_t(4) << 20;
 
+// Whether a copy of `bytes` from or to the caller's memory p goes through the staging. Page-locked
+// memory needs none: the copy is one DMA (rays and hits in page-locked memory, staged and directly:
+// 300,001 rays 0.94 to 1.0 and 0.43 ms a call, 2,000,000 rays 4.7 and 2.3 ms).
+bool wants_staging(const void* p, size_t bytes) {
+    if (bytes < kCopyStaged) return false;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
 int staged_copy(int device, cudaStream_t st, void* dev, void* host, size_t bytes, bool to_device) {
     const int chunks = int((bytes + kCopyChunk - 1) / kCopyChunk);
     const unsigned hw = std::max(2u, std::thread::hardware_concurrency());
@@ -1291,7 +1304,7 @@ int trace_direct(lux_ctx* C, const float* rays, int n, int mode, int iter, uint3
     volatile int* failed = word;
     int copied = 0;
     if (failed) *failed = 0;
-    if (in >= kCopyStaged) {
+    if (wants_staging(rays, in)) {
         if (int rc = staged_copy(C->device, C->stream, sc.rays, const_cast<float*>(rays), in, true)) return rc;
     } else {
         LUX_CUDA(cudaMemcpyAsync(sc.rays, rays, in, cudaMemcpyHostToDevice, C->stream));
@@ -1301,7 +1314,7 @@ int trace_direct(lux_ctx* C, const float* rays, int n, int mode, int iter, uint3
     cudaError_t e = launch_trace_ext(C->S, C->W, sc.rays, sc.hits, n, mode, iter, sc.cursor, word ? word : dev_word, C->stream);
     int rc = e == cudaSuccess ? LUX_OK : fail(LUX_ERR_CUDA, cudaGetErrorString(e));
     if (!rc) {
-        if (out >= kCopyStaged) {
+        if (wants_staging(hits, out)) {
             rc = staged_copy(C->device, C->stream, sc.hits, hits, out, false);
         } else {
             e = cudaMemcpyAsync(hits, sc.hits, out, cudaMemcpyDeviceToHost, C->stream);

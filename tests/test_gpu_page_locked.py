@@ -80,3 +80,31 @@ def test_call_without_page_locked_memory_for_the_error_word(renderer, n):
         left = fail_pinned(0)
     assert np.array_equal(got, want)
     assert left < MANY
+
+
+def page_locked(shape, dtype):
+    import torch
+    return torch.empty(shape, dtype=dtype, pin_memory=True).numpy()
+
+
+@pytest.mark.parametrize("n", [131_071, 131_072, 209_715, 209_716])
+@pytest.mark.parametrize("rays_locked,hits_locked", [(True, True), (True, False), (False, True)])
+def test_page_locked_buffers_are_not_staged(renderer, n, rays_locked, hits_locked):
+    # the library asks for one block for the error word, and for one per buffer that it stages:
+    # pageable ones of 4 MB (131,072 rays, 209,716 hits) and more
+    import torch
+    rays = some_rays(n)
+    want = renderer.trace_rays(rays, 0, 1)
+    hits = np.zeros((n, 5), np.uint32)
+    if rays_locked:
+        src, rays = rays, page_locked((n, 8), torch.float32)
+        rays[:] = src
+    if hits_locked:
+        hits = page_locked((n, 5), torch.int32).view(np.uint32)
+    fail_pinned(MANY)
+    try:
+        rc = lx.lib().lux_trace_rays(renderer._h, lx.ptr(rays), n, 0, 1, lx.ptr(hits, C.c_uint32))
+    finally:
+        asked = MANY - fail_pinned(0)
+    assert rc == 0 and np.array_equal(hits, want)
+    assert asked == 1 + (not rays_locked and n >= 131_072) + (not hits_locked and n >= 209_716)
