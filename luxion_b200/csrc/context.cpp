@@ -1274,7 +1274,9 @@ int staged_copy(int device, cudaStream_t st, void* dev, void* host, size_t bytes
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[k]);
             if (e == cudaSuccess) std::memcpy(static_cast<char*>(host) + at(c), slot[k], len(c));
         }
-        // the staging goes back to the pool once its last copies are done
+        // The staging goes back to the pool once its last copies are done. After a failure the last
+        // copy may be one that no event follows.
+        if (e != cudaSuccess) cudaStreamSynchronize(st);
         for (int j = 0; j < 2; ++j)
             if (ev[j]) {
                 const cudaError_t w = cudaEventSynchronize(ev[j]);
