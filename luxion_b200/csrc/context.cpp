@@ -34,7 +34,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <tuple>
 #include <vector>
@@ -1289,7 +1288,7 @@ int staged_copy(int device, cudaStream_t st, void* dev, void* host, size_t bytes
     int started = 1;
     try {
         for (; started < nt; ++started) th[started] = std::thread(work, started);
-    } catch (const std::system_error&) {  // no thread to be had: its chunks are moved here
+    } catch (...) {  // no thread, or no memory for one: its chunks are moved here
     }
     work(0);
     for (int t = started; t < nt; ++t) work(t);

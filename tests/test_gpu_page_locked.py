@@ -108,3 +108,37 @@ def test_page_locked_buffers_are_not_staged(renderer, n, rays_locked, hits_locke
         asked = MANY - fail_pinned(0)
     assert rc == 0 and np.array_equal(hits, want)
     assert asked == 1 + (not rays_locked and n >= 131_072) + (not hits_locked and n >= 209_716)
+
+
+class NoThreads:
+    """No thread can be started meanwhile: the default stack is larger than the address space."""
+
+    def __enter__(self):
+        self.libc, self.old, new = C.CDLL(None), C.create_string_buffer(256), C.create_string_buffer(256)
+        assert self.libc.pthread_getattr_default_np(self.old) == 0
+        assert self.libc.pthread_attr_init(new) == 0
+        assert self.libc.pthread_attr_setstacksize(new, C.c_size_t(1 << 47)) == 0
+        assert self.libc.pthread_setattr_default_np(new) == 0
+
+    def __exit__(self, *exc):
+        assert self.libc.pthread_setattr_default_np(self.old) == 0
+
+
+@pytest.mark.parametrize("staging", [True, False], ids=["staging", "no-staging"])
+@pytest.mark.parametrize("threads", [True, False], ids=["threads", "no-threads"])
+@pytest.mark.parametrize("n", [131_073, 262_145])
+def test_large_batches_without_threads_or_staging(renderer, n, threads, staging):
+    rays = some_rays(n)
+    step = 50_021
+    want = np.concatenate([renderer.trace_rays_static(rays[i:i + step], 0, 1) for i in range(0, n, step)])
+    renderer.trace_rays(rays, 0, 1)
+    fail_pinned(0 if staging else MANY)
+    try:
+        if threads:
+            got = renderer.trace_rays(rays, 0, 1)
+        else:
+            with NoThreads():
+                got = renderer.trace_rays(rays, 0, 1)
+    finally:
+        fail_pinned(0)
+    assert np.array_equal(got, want)
