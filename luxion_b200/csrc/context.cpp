@@ -1002,7 +1002,8 @@ int finish_stats(lux_ctx* C, int nwaves, int n_iter, const Spans* sp, int steps)
     }
     C->stats.launches_camera += nwaves;
     C->stats.launches_accum += nwaves;
-    C->stats.launches_trace += steps * (nee ? 2 : 1) + (whole_paths(C) ? tail_attempts(depth) : 0);
+    const int chunks = (nwaves + kWaveTab - 1) / kWaveTab;  // each with a last wave to hand over
+    C->stats.launches_trace += steps * (nee ? 2 : 1) + (whole_paths(C) ? chunks * tail_attempts(depth) : 0);
     C->stats.launches_shade += steps;
     if (sp) {
         for (size_t i = 1; i < sp->marks.size(); ++i) {
