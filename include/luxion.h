@@ -351,6 +351,13 @@ int lux_bvh8_build(const float* boxes, const int* tree_begin, int num_trees, int
  * rays as in lux_trace_rays; keys: n u32. Host buffers. */
 int lux_morton_keys(lux_ctx* ctx, const float* rays, int n, uint32_t* keys);
 
+/* The ray sort of a wave (src/pathtrace.cu:182) on caller rays, for the parity test: the queue
+ * 0 .. n-1 is sorted stably by the rays' Morton keys, once for each bounce 0 .. bounce, as the
+ * bounces of one wave are. order: the last bounce's queue, n ints; keys: its keys in that order,
+ * n u32. The context has ray sorting on and a wave of at least n paths; the call uses the wave's
+ * buffers. Host buffers. */
+int lux_morton_sort(lux_ctx* ctx, const float* rays, int n, int bounce, uint32_t* keys, int* order);
+
 /* One bounce of the wavefront on caller state, for the shade parity test. The caller gives
  * n paths (path state, 24 floats each, layout LUX_PS_*) and the traced hits for them
  * (10 words each: radiance hit, then shadow hit / occlusion), the bounce depth after the

@@ -56,6 +56,7 @@ SIGNATURES = {
     "lux_trace_rays_static": (C.c_int, [_P, c_float_p, C.c_int, C.c_int, C.c_int, c_u32_p]),
     "lux_device_alloc_count": (C.c_int64, []),
     "lux_morton_keys": (C.c_int, [_P, c_float_p, C.c_int, c_u32_p]),
+    "lux_morton_sort": (C.c_int, [_P, c_float_p, C.c_int, C.c_int, c_u32_p, c_int_p]),
     "lux_bvh8_build": (C.c_int, [c_float_p, c_int_p, C.c_int, C.c_int, C.c_void_p, C.c_int, c_u32_p, c_u32_p, c_int_p,
                                  c_int_p]),
     "lux_shade_step": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, c_float_p, C.c_int, c_u32_p, c_int_p, c_int_p]),
@@ -355,6 +356,14 @@ class Renderer:
         keys = np.zeros(rays.shape[0], np.uint32)
         _check(lib().lux_morton_keys(self._h, ptr(rays), rays.shape[0], ptr(keys, C.c_uint32)))
         return keys
+
+    def morton_sort(self, rays: np.ndarray, bounce: int = 0):
+        """(keys, order) of the wave's ray sort over the queue 0 .. n-1; needs ray_sorting."""
+        rays = np.ascontiguousarray(rays, np.float32)
+        n = rays.shape[0]
+        keys, order = np.zeros(n, np.uint32), np.zeros(n, np.int32)
+        _check(lib().lux_morton_sort(self._h, ptr(rays), n, bounce, ptr(keys, C.c_uint32), ptr(order, C.c_int)))
+        return keys, order
 
     def shade_step(self, paths: np.ndarray, hits: np.ndarray, it: int, depth: int, compact: int = 1):
         paths = np.ascontiguousarray(paths, np.float32).copy()

@@ -32,7 +32,9 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -1894,6 +1896,36 @@ int lux_morton_keys(lux_ctx* C, const float* rays, int n, uint32_t* keys) {
     LUX_CUDA(cudaMemcpyAsync(keys, dk, size_t(n) * sizeof(uint32_t), cudaMemcpyDeviceToHost, C->stream));
     LUX_CUDA(cudaStreamSynchronize(C->stream));
     return LUX_OK;
+}
+
+int lux_morton_sort(lux_ctx* C, const float* rays, int n, int bounce, uint32_t* keys, int* order) {
+    if (!C || n < 0 || bounce < 0 || bounce >= kMaxDepth || (n > 0 && (!rays || !keys || !order)))
+        return fail(LUX_ERR_INVALID, "bad arguments");
+    if (!C->opt.ray_sorting) return fail(LUX_ERR_STATE, "the context was made without ray sorting");
+    if (n > C->W.max_paths) return fail(LUX_ERR_INVALID, "more rays than a wave has paths");
+    if (n == 0) return LUX_OK;
+    LUX_CUDA(cudaSetDevice(C->device));
+    cudaStream_t st = C->stream;
+    DevWave& W = C->W;
+    const size_t q = size_t(n) * sizeof(int), row = 8 * sizeof(float), half = sizeof(float4);
+    std::unique_ptr<int[]> iota(new (std::nothrow) int[size_t(n)]);
+    if (!iota) return fail(LUX_ERR_OOM, "host allocation failed");
+    for (int i = 0; i < n; ++i) iota[i] = i;
+    LUX_CUDA(cudaMemsetAsync(W.ctr, 0, sizeof(WaveCounters), st));
+    LUX_CUDA(clear_sort_counters(C->sort_temp, st));
+    LUX_CUDA(cudaMemcpy2DAsync(W.s0, half, rays, row, half, size_t(n), cudaMemcpyHostToDevice, st));
+    LUX_CUDA(cudaMemcpy2DAsync(W.s1, half, rays + 4, row, half, size_t(n), cudaMemcpyHostToDevice, st));
+    for (int b = 0; b <= bounce; ++b) {
+        LUX_CUDA(cudaMemcpyAsync(W.queue[b & 1], iota.get(), q, cudaMemcpyHostToDevice, st));
+        LUX_CUDA(cudaMemcpyAsync(&W.ctr->count[b], &n, sizeof(int), cudaMemcpyHostToDevice, st));
+        LUX_CUDA(launch_morton_sort(C->S, W, b, C->sort_temp, C->sort_temp_bytes, st));
+    }
+    int err = 0;
+    LUX_CUDA(cudaMemcpyAsync(keys, W.keys, size_t(n) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    LUX_CUDA(cudaMemcpyAsync(order, W.queue[bounce & 1], q, cudaMemcpyDeviceToHost, st));
+    LUX_CUDA(cudaMemcpyAsync(&err, &W.ctr->error, sizeof(int), cudaMemcpyDeviceToHost, st));
+    LUX_CUDA(cudaStreamSynchronize(st));
+    return err ? wave_error(err) : LUX_OK;
 }
 
 int lux_shade_step(lux_ctx* C, int iter, int depth, int compact, float* paths, int n, const uint32_t* hits,
