@@ -4,8 +4,9 @@
 // and, in its active build, hands the triangles to OptiX, which builds on the device
 // (src/myoptix/optix_accel.cpp:40-106). Here every BLAS and the TLAS are built by kernels:
 // a binned-SAH binary tree (32 bins per axis, cost SA(L)*nL + SA(R)*nR), level by level for
-// nodes of more than 32 primitives and one warp per subtree below that, then collapsed into
-// 8-wide nodes with quantised child boxes, level by level. The arithmetic is the host
+// nodes of more than 1024 primitives, one block per subtree from there down to 32 and one warp
+// per subtree below that, then collapsed into 8-wide nodes with quantised child boxes, one launch
+// a level. The arithmetic is the host
 // builder's (bvh_build.cpp) operation for operation, so both produce the same nodes bit for bit.
 #pragma once
 

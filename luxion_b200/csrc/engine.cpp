@@ -663,6 +663,7 @@ int step_pipelined(lux_engine* E, int* done_jobs, int* idle) {
             ++G.n;
         }
         if (G.n == 0) break;
+        // (the youngest wave is at a multiple of kStepBounces, and not in its first step: bounce 3)
         if (drain && try_tail(E->flight.back().bounce, E->flight.back().depth))
             LUX_CUDA(launch_paths(E->S, E->W, E->dopt, G, kMaxDepth, path_limit(kTailPerLane), st));
         LUX_CUDA(launch_trace_segs(E->S, E->W, G, 0, nee, st, E->trace_blocks));

@@ -54,13 +54,19 @@ cudaError_t launch_paths(const DevScene& S, const DevWave& W, const DevOptions& 
                          cudaStream_t st);
 int path_grid_blocks();
 // Waves of at most kWholePerLane paths per lane of the whole-path kernel's grid (284k on 148 SMs)
-// run in it from the camera on. Above, the wavefront's full warps win: 0.81 against 1.18 ms for
-// 228k paths (477k triangles) and 0.35 against 0.53 for 66k (Cornell box), but 1.65 against 1.12 ms
-// for 367k (842k triangles). A larger wave hands over before one of the bounces 1 to kTailLast once
-// at most kTailPerLane paths per lane are left (114k) and two bounces or more are to come: a frame
-// of 2.07M paths, 1M triangles, depth 12 takes 4.18 ms instead of 5.34, while handing over at
-// twice that many took 5 to 20 % longer in 700k-triangle scenes. An attempt that finds more paths
-// left costs an empty launch.
+// run in it from the camera on. Above, the wavefront's full warps win. One sample, depth 8, both light
+// samplings (the box: emitters), ms a wave as a wavefront and whole (medians of 41):
+//   paths            150k        200k        250k        284k        350k        450k
+//   Cornell box   0.60 0.41   0.61 0.48   0.66 0.55   0.66 0.60   0.71 0.71   0.81 0.88
+//   50k triangles 0.72 0.46   0.79 0.54   0.83 0.63   0.85 0.68   0.90 0.79   0.98 0.96
+//   400k          1.16 0.81   1.25 0.97   1.34 1.11   1.38 1.24   1.44 1.42   1.56 1.72
+//   1M            1.48 1.29   1.60 1.56   1.70 1.84   1.75 2.03   1.92 2.42   2.18 2.99
+// At 284k it still wins by 9 to 20 % up to 400k triangles and loses 16 % at 1M, where the two meet at
+// 210k; without light sampling the figures stand alike (284k: 0.35 0.34, 0.51 0.43, 0.89 0.81, 1.08 1.30).
+// A larger wave hands over before one of the bounces 1 to kTailLast once at most kTailPerLane paths per
+// lane are left (114k) and two bounces or more are to come: a frame of 2.07M paths, 1M triangles, depth 12
+// took 4.18 ms instead of 5.34 when it came, while handing over at twice that many took 5 to 20 %
+// longer in 700k-triangle scenes. An attempt that finds more paths left costs an empty launch.
 constexpr int kWholePerLane = 5;
 constexpr int kTailPerLane = 2;
 constexpr int kTailLast = 3;

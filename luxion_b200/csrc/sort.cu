@@ -113,6 +113,9 @@ __global__ void __launch_bounds__(kSortThreads) k_keys(DevScene S, DevWave W, in
         W.keys[i] = key;
         for (int p = 0; p < kPasses; ++p) {
             // lanes of one digit value add together: the keys of a tile share their upper digits
+            // (the lanes that are together here: with rounds of whole warps and a digit of its own for
+            // lanes past the end, the sorting of an 800x600, 4 spp, depth 8 render took 0.574 instead of
+            // 0.557 ms)
             const int dg = (key >> (8 * p)) & 0xff;
             const unsigned peers = __match_any_sync(__activemask(), dg);
             if (__ffs(peers) - 1 == int(threadIdx.x & 31)) atomicAdd(&h[p][dg], __popc(peers));

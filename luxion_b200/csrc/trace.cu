@@ -1,4 +1,4 @@
-// trace.cu -- ray traversal of the two-level compressed 8-wide BVH on sm_100a.
+// trace.cu -- ray traversal of the compressed 8-wide BVH, of two levels or one, on sm_100a.
 //
 // Replaces the reference's OptiX launch (src/pathtrace.cu:238-258, device programs in
 // src/optixshaders/optix_triangle.cu:52-366) and its disabled software path
@@ -13,7 +13,7 @@
 //    thread, conflict-free) and spills deeper entries to local memory;
 //  * node groups / triangle groups as in Ylitie et al. 2017: a stack entry is a node's
 //    remaining internal-child hits (ordered by ray octant) or a set of leaf records;
-//  * two levels: the TLAS is traversed with the world ray; a TLAS leaf pushes a marker and
+//  * two-level layout: the TLAS is traversed with the world ray; a TLAS leaf pushes a marker and
 //    continues in the instance's BLAS with the object-space ray the reference uses
 //    (inverseTransform * (o,1), (d,0), src/intersections/mesh_isect.cu:15-16);
 //  * the triangle test is the reference's Moller-Trumbore (mesh_isect.cu:78-137) with every

@@ -272,7 +272,7 @@ struct Lane {
 
 // MODE: 0 radiance, 1 DL shadow, 2 env occlusion (any hit), 3 BVH heatmap; -1: `any` says at run
 // time whether any hit ends the ray (one copy of the code for both kinds of ray).
-// KEY: gives the pixel and iteration that key a ray's alpha-blend hash, from Lane::key.
+// KEY: gives the pixel and iteration that key a ray's alpha-blend hash, from Lane::item.
 template <int MODE, bool SINGLE, int BLOCK, class KEY>
 struct Tracer {
     const DevScene& S;
